@@ -132,17 +132,23 @@ typedef struct {
     double work_relabel_factor;   /* relabel after this many node visits per
                                      free node since the last one; default 3
                                      (one launch per step); persistent: 2 below
-                                     500k free nodes, 1 below 10M, else 0.5 */
+                                     500k free nodes, 1 below 10M, else 0.5, and
+                                     earlier once a discharge phase has taken
+                                     1.2 times the relabel before it without
+                                     halving its active nodes */
     int32_t engine;               /* 0 auto (persistent when the device supports
                                      cooperative launch), 1 one launch per BFS
                                      level / round, 2 persistent */
     int32_t chain_hops;           /* persistent engine: nodes one thread may
-                                     discharge in a row in one round (1 = no
-                                     chaining; default 4) */
+                                     discharge in a row in one round, instead of
+                                     the round's block sub-levels (default 1 = no
+                                     chaining) */
     int32_t chain_max_active;     /* ... only in rounds with at most this many
-                                     active nodes (default by graph size: 131072
-                                     below 1.5M free nodes, 32768 below 2M,
-                                     else 4096) */
+                                     active nodes (default 131072); without
+                                     chaining such rounds run 16 sub-levels,
+                                     wider ones 4.  max_rounds below 16384
+                                     counts rounds of one discharge per queued
+                                     node and turns the sub-levels off */
     int32_t bfs_bottom_up;        /* persistent engine: 1 = direction-optimizing
                                      global relabels (bottom-up steps over the
                                      nodes the previous relabel reached and this
@@ -250,10 +256,7 @@ typedef struct {
  * finds no active node in it (its labels are then final and later relabels
  * skip it).  Unless options set chain_hops, chain_max_active, blocks_per_sm or
  * work_relabel_factor, the batch takes the batch tuning table's entry for its
- * size bucket (gpupr_autotune_batch); without one, a batch of at least 16
- * graphs averaging under 1.5M tets solves with 8 chained hops in rounds of up
- * to 131072 active nodes on 3 blocks per SM (the setting that suits small
- * graphs; the union's own size would pick another).
+ * size bucket (gpupr_autotune_batch); without one, the union's own size rule.
  */
 gpupr_status gpupr_graph_cut_batch(uint32_t n_graphs, const uint64_t* tet_offsets,
                                    const uint64_t* vertex_offsets, const double* vertices,

@@ -424,15 +424,9 @@ void prepare_batch(uint32_t G, const uint64_t* toff, const uint64_t* voff, const
 
 // The options of a batch's solve: the caller's fields where set; else the
 // batch tuning table's entry for the batch's size class (free nodes per
-// graph); else, for a union of at least 16 graphs averaging under 1.5M tets,
-// 8 chained hops in rounds of up to 131072 active nodes on 3 blocks per SM.
-// That rule comes from B200 measurements with 64 graphs of 50k-4M tets
-// (56.5M in all, mean 0.9M; median solve of 9 alternating runs): 73.3 ->
-// 54.7 ms on one seeded batch, 86.3 -> 90.7 ms on another, against the
-// union's own size rule; a single 5M-tet graph ran 3x slower with these
-// settings, hence the mean-size bound.
-gpupr_solve_options batch_options(const gpupr_solve_options* options, uint32_t G, uint64_t N,
-                                  uint64_t free_n)
+// graph); else the union's own size rule (64 graphs of 50k-4M tets, mean of
+// three seeds: 61.7 ms, 70.0 ms on 3 blocks per SM).
+gpupr_solve_options batch_options(const gpupr_solve_options* options, uint32_t G, uint64_t free_n)
 {
     gpupr_solve_options o{};
     if (options) o = *options;
@@ -445,10 +439,6 @@ gpupr_solve_options batch_options(const gpupr_solve_options* options, uint32_t G
         o.work_relabel_factor = e.work_factor;
         o.chain_hops = e.chain_hops;
         o.chain_max_active = e.chain_max_active;
-    } else if (G >= 16u && N / G < 1500000ull) {
-        o.chain_hops = 8;
-        o.chain_max_active = 131072;
-        o.blocks_per_sm = 3;
     }
     return o;
 }
@@ -497,7 +487,7 @@ void run_graph_cut_batch(uint32_t G, const uint64_t* toff, const uint64_t* voff,
         st->native_total_seconds = seconds_since(all0);
         return;
     }
-    const gpupr_solve_options bo = batch_options(options, G, N, info.free_n);
+    const gpupr_solve_options bo = batch_options(options, G, info.free_n);
     SolveOptions opt = resolve_options(&bo, 8, 1024, 2000000ull);
     opt.max_blocks_per_sm = max_blocks_per_sm;
     SolveWorkspace w;
@@ -596,7 +586,7 @@ TuneEntry run_autotune_batch(uint32_t G, const uint64_t* toff, const uint64_t* v
                               [&](const TuneEntry& e) { return e.size_class == size_class((uint32_t)mean_free); }),
                keep.end());
     batch_tune_replace(keep);
-    const gpupr_solve_options base = batch_options(nullptr, G, toff[G], pb.info.free_n);
+    const gpupr_solve_options base = batch_options(nullptr, G, pb.info.free_n);
     TuneEntry best = two_stage_tune(pb.g, &pb.segs, base, local_steps, reps, s);
     best.size_class = size_class((uint32_t)mean_free);
     batch_tune_store(best);

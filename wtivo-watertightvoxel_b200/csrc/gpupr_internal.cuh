@@ -71,6 +71,8 @@ struct Ctl {
     // <= 131072, larger) and block 0's time in each class
     uint32_t dround_cnt[3];
     unsigned long long dround_ns[3];
+    uint32_t stop_round;     // persistent engine: the discharge phase ends after this round
+    uint32_t pad1;
 };
 
 // Nodes per tile of a tiled relabel (a power of two; the persistent engine
@@ -112,7 +114,11 @@ struct SolveView {
     int local_steps;
     int chain_hops;                     // nodes one thread may discharge in a row in
                                         // one round (<= 1: no chaining) ...
-    uint32_t chain_max_active;          // ... in rounds of at most this many nodes
+    uint32_t chain_max_active;          // ... in rounds of at most this many nodes (the
+                                        // short rounds)
+    int dis_levels;                     // persistent engine: levels of a discharge round of at
+                                        // most chain_max_active nodes (1: no sub-levels) ...
+    int dis_levels_wide;                // ... and of a wider one
     int bfs_block_levels;               // persistent engine: > 1 = BFS steps expand that many
                                         // levels per block from its shared stage (0: chains)
     int bfs_hops;                       // nodes one thread may label in a row in one

@@ -10,8 +10,10 @@
 //    other engine launches one kernel per step, reading queue sizes from a
 //    device control block (ring counters), with the host checking the state
 //    once per batch of steps.
-//  * Chained discharge: the thread that takes ownership of a neighbour's
-//    excess may discharge it at once, so excess moves several hops a round.
+//  * Discharge rounds in block sub-levels: after its share of the active
+//    queue a block discharges the nodes it activated itself, level after
+//    level, from its shared-memory stage, so one grid barrier covers up to 16
+//    hops; short lists give each node four lanes, one per arc.
 //  * Label-correcting BFS steps (persistent engine): labels are lowered by
 //    atomicMin, and after expanding its share of the frontier each block
 //    expands the nodes it labelled itself for up to 16 levels from its
@@ -310,6 +312,23 @@ __device__ __forceinline__ uint32_t queue_index(uint32_t it, uint32_t cnt)
     return (it * gridDim.x + blockIdx.x) * DTPB + threadIdx.x;
 }
 
+// Staged nodes of a block up to which a sub-level gives each node four lanes
+// (discharge_quad, bfs_expand_quad).  With a thread per node a short list
+// leaves one or two warps walking the node's four slots one after the other,
+// and a sub-level lasts as long as that instruction chain; four lanes do the
+// slots at once (a 200k-node integer graph: 2.7 -> 1.8 ms, an 8M-tet open box
+// 26.6 -> 18.6 ms with the same schedule).  Above three passes of 64 nodes the
+// threads are better spent on more nodes at a time.
+constexpr uint32_t QUAD_MAX = 192u;
+
+// Queue index of a thread's node in pass `it` when four lanes share a node:
+// eight entries per warp, dealt round-robin over the blocks.
+__device__ __forceinline__ uint32_t quad_index(uint32_t it)
+{
+    const uint32_t chunk = (it * (DTPB / 32) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x;
+    return chunk * 8u + ((threadIdx.x & 31u) >> 2);
+}
+
 // The active queue after a BFS of the persistent engine: every node with a
 // label below n and positive excess, appended in node order by one streaming
 // pass (12 bytes a node) instead of a random excess load for each node the
@@ -367,6 +386,15 @@ __device__ __forceinline__ void active_sweep_body(const SolveView& g, uint32_t* 
 __device__ __forceinline__ uint32_t prefetch_entry(const uint32_t* in, uint32_t n)
 {
     const uint32_t i = queue_index(0, 0u);
+    uint32_t v = 0;
+    if (i < n) asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(in + i) : "memory");
+    return v;
+}
+
+// The same for a pass of four lanes per node (quad_index(0)).
+__device__ __forceinline__ uint32_t prefetch_quad(const uint32_t* in, uint32_t n)
+{
+    const uint32_t i = quad_index(0);
     uint32_t v = 0;
     if (i < n) asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(in + i) : "memory");
     return v;
@@ -498,6 +526,11 @@ __global__ void __launch_bounds__(DTPB) k_bfs_level(SolveView g, uint32_t L)
     const unsigned long long vs = warp_block_sum(visits, s_red);
     if (threadIdx.x == 0 && vs) atomicAdd(&ctl->bfs_visits, vs);
 }
+
+// s_m[SUB..SUB+2]: a block's sub-level counts, a ring (the level being read,
+// the one being filled, the one being cleared), so that a sub-level needs one
+// block barrier.  All three are 0 between passes.
+constexpr uint32_t SUB = 12u;
 
 struct Work {
     unsigned long long visits = 0, pushes = 0, relabels = 0, sink = 0;
@@ -914,6 +947,64 @@ __device__ __forceinline__ void bfs_expand_one(const SolveView& g, uint32_t u, u
     }
 }
 
+// Appends this lane's entries to the stage: u where `want` holds, v where
+// `want2` does; every lane of the warp calls it: one shared atomic per warp.
+__device__ __forceinline__ void stage_push_warp(const SolveView& g, const Stage& st, bool want, uint32_t u,
+                                                bool want2 = false, uint32_t v = 0u)
+{
+    const unsigned b1 = __ballot_sync(0xffffffffu, want);
+    const unsigned b2 = __ballot_sync(0xffffffffu, want2);
+    if (!(b1 | b2)) return;
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    uint32_t base = 0;
+    if (lane == 0u) base = atomicAdd(st.cnt, (uint32_t)(__popc(b1) + __popc(b2)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    uint32_t idx = base + (uint32_t)__popc(b1 & below);
+    if (want) {
+        if (idx < st.cap) {
+            st.buf[idx] = u;
+        } else {
+            const uint32_t pos = atomicAdd(st.gcnt, 1u);
+            if (pos < g.n) st.out[pos] = u;
+            else raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+        }
+    }
+    if (want2) {
+        idx = base + (uint32_t)(__popc(b1) + __popc(b2 & below));
+        if (idx < st.cap) {
+            st.buf[idx] = v;
+        } else {
+            const uint32_t pos = atomicAdd(st.gcnt, 1u);
+            if (pos < g.n) st.out[pos] = v;
+            else raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+        }
+    }
+}
+
+// bfs_expand_one by four lanes, one per slot (in-arc masks only): the warp
+// holds eight nodes, `valid` where this lane's node exists.
+__device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, uint32_t u, uint32_t L,
+                                                bool exact, const Stage& st, bool propagate,
+                                                unsigned long long& visits, uint32_t* s_m)
+{
+    const uint32_t k = threadIdx.x & 3u;
+    bool want = false;
+    int nb = 0;
+    if (valid) {
+        const uint32_t hu = exact ? L : ldcg(g.height + u);
+        nb = __ldg(reinterpret_cast<const int*>(g.nbr) + (size_t)u * 4u + k);
+        const uint32_t m = __ldcg(g.inm + u);
+        if (k == 0u) ++visits;
+        const uint32_t cand = hu + 1u;
+        if (((m >> k) & 1u) && ldcg(g.height + nb) > cand) {
+            const uint32_t old = atomicMin(g.height + nb, cand);
+            if (g.bottom_up && old == UNVIS) atomicAdd(&s_m[6], 1u);   // a first label
+            want = old > cand && (old == UNVIS || propagate);
+        }
+    }
+    stage_push_warp(g, st, want, (uint32_t)nb);
+}
+
 // A BFS step of the persistent engine with block sub-levels (option
 // bfs_block_levels = K > 1): each block expands its share of the frontier
 // (level L), then, without a grid barrier, the nodes it labelled itself, for
@@ -935,37 +1026,54 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
     uint32_t* out = (L & 1) ? g.fr[0] : g.fr[1];
     uint32_t* gcnt = &ctl->bfs_cnt[(L + 1) % 3];
     const uint32_t half = stage_cap / 2u;
-    for (uint32_t it = 0; it * (gridDim.x * DTPB) < cnt; ++it) {
+    const bool quads = g.inm && cnt <= SPREAD_MAX;
+    const uint32_t per_pass = gridDim.x * (quads ? DTPB / 4u : (uint32_t)DTPB);
+    for (uint32_t it = 0; it * per_pass < cnt; ++it) {
         uint32_t* cur = s_fr;
         uint32_t* nxt = s_fr + half;
-        {
-            const Stage st{cur, &s_m[0], half, gcnt, out};
+        const Stage st0{cur, &s_m[SUB], half, gcnt, out};
+        if (quads) {
+            const uint32_t i = quad_index(it);
+            const bool valid = i < cnt;
+            const uint32_t u = it == 0 ? first : (valid ? __ldcg(in + i) : 0u);
+            if (__any_sync(0xffffffffu, valid)) bfs_expand_quad(g, valid, u, L, exact, st0, propagate, visits, s_m);
+        } else {
             const uint32_t i = queue_index(it, cnt);
             if (i < cnt) {
-                const uint32_t u = (it == 0 && cnt <= SPREAD_MAX) ? first : __ldcg(in + i);
-                bfs_expand_one(g, u, exact ? L : ldcg(g.height + u), st, propagate, visits, s_m);
+                const uint32_t u = __ldcg(in + i);
+                bfs_expand_one(g, u, exact ? L : ldcg(g.height + u), st0, propagate, visits, s_m);
             }
         }
         __syncthreads();
+        uint32_t last = 0;   // ring slot of the last sub-level's count
         for (int k = 1; k < levels; ++k) {
-            const uint32_t c = min(s_m[0], half);
-            __syncthreads();   // every thread has read the count
+            const uint32_t c = min(s_m[SUB + last], half);
             if (c == 0u) break;
-            if (threadIdx.x == 0) s_m[0] = 0u;
-            __syncthreads();
-            const Stage st{nxt, &s_m[0], half, gcnt, out};
-            for (uint32_t j = threadIdx.x; j < c; j += DTPB) {
-                const uint32_t u = cur[j];
-                bfs_expand_one(g, u, ldcg(g.height + u), st, propagate, visits, s_m);
+            const uint32_t nx = last == 2u ? 0u : last + 1u;
+            // the slot after next was read before the last block barrier
+            if (threadIdx.x == 0) s_m[SUB + (nx == 2u ? 0u : nx + 1u)] = 0u;
+            const Stage st{nxt, &s_m[SUB + nx], half, gcnt, out};
+            if (g.inm && c <= QUAD_MAX) {
+                // a warp without a node has nothing to do
+                for (uint32_t j0 = (threadIdx.x >> 5) * 8u; j0 < c; j0 += DTPB / 4u) {
+                    const uint32_t j = j0 + ((threadIdx.x & 31u) >> 2);
+                    const bool valid = j < c;
+                    bfs_expand_quad(g, valid, valid ? cur[j] : 0u, 0u, false, st, propagate, visits, s_m);
+                }
+            } else {
+                for (uint32_t j = threadIdx.x; j < c; j += DTPB) {
+                    const uint32_t u = cur[j];
+                    bfs_expand_one(g, u, ldcg(g.height + u), st, propagate, visits, s_m);
+                }
             }
             __syncthreads();
             uint32_t* tmp = cur;
             cur = nxt;
             nxt = tmp;
+            last = nx;
         }
         if (threadIdx.x == 0) {
-            s_m[2] = min(s_m[0], half);
-            s_m[0] = 0;
+            s_m[2] = min(s_m[SUB + last], half);
             s_m[4] = s_m[2] ? atomicAdd(gcnt, s_m[2]) : 0u;
             if (g.bottom_up && s_m[6]) {
                 atomicAdd(&ctl->lab_cnt[(L + 1) % 3], s_m[6]);
@@ -974,6 +1082,7 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
         }
         __syncthreads();
         flush_stage(cur, s_m[2], s_m[4], out, g.n, ctl);
+        if (threadIdx.x < 3) s_m[SUB + threadIdx.x] = 0u;
         __syncthreads();
     }
 }
@@ -997,6 +1106,34 @@ constexpr int BFS_BLOCK_LEVELS = 16;
 // (relabels 36.3 -> 35.0 ms), 3M-tet torus 1.83 -> 1.81 ms, 8M-tet open box
 // 12.8 -> 12.6 ms; 15 bytes less workspace per node.
 constexpr bool BFS_IN_ARC_MASKS_DEFAULT = true;
+// Sub-levels of a discharge round (discharge_body): a block discharges its
+// share of the active queue and then, without a grid barrier, the nodes those
+// discharges made or left active, level after level.  A short round is a chain
+// of memory round trips, so many levels share one barrier; in a wide round the
+// nodes of other blocks fall behind and excess that would have merged is moved
+// twice, so few do.  Measured on B200 (mean of three seeds, solve time, 8 / 16 /
+// 32 levels in short rounds): a 200k-node integer graph 1.80 / 1.74 / 2.12 ms,
+// an 8M-tet open box 19.9 / 18.6 / 18.9 ms; wide rounds of 1 / 4 / 8 / 12
+// levels: an 80M-tet knot 96 / 78 / 90 / 93 ms, 64 graphs of 50k-4M tets 69 /
+// 63 / 62 / 62 ms.  Rounds of up to 32768, 65536, 131072 or 262144 active nodes
+// counted as short: within 3% of each other on all of them.
+constexpr int DIS_LEVELS = 16;
+constexpr int DIS_LEVELS_WIDE = 4;
+constexpr uint32_t DIS_NARROW_MAX = 131072u;
+
+// When a discharge phase ends (persistent engine, besides the work budget and
+// the round cap): after RELABEL_TIME_RATIO times what the relabel before it
+// took, unless the active nodes fell to 1/RELABEL_GAIN in that time, which
+// buys the phase as much time again.  Time spent on relabels and on discharge
+// stays balanced whatever the graph's size and shape: counting rounds or
+// visits alone left a 200k-node integer graph in 1,024 rounds of a few stuck
+// nodes (16.7 ms, 1.8 ms with this rule), and a 12M-node one needs no relabel
+// in its long tail of shrinking rounds (10.6 ms without the second half of the
+// rule, 6.7 ms with it).  Ratios of 0.8 / 1.2 / 1.5 / 2: 3.2M-tet sphere 3.7 /
+// 4.1 / 4.0 / 4.8 ms, 8M-tet box 22.5 / 19.4 / 19.3 / 19.4 ms.
+constexpr float RELABEL_TIME_RATIO = 1.2f;
+constexpr float RELABEL_GAIN = 2.0f;
+
 // Free nodes from which the persistent engine relabels by tiles by default.
 constexpr uint32_t RELABEL_TILES_DEFAULT_MIN = 0xFFFFFFFFu;
 
@@ -1154,8 +1291,10 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
     const int4 nb4 = __ldg(g.nbr + v);
     const uint4 r4 = __ldcg(reinterpret_cast<const uint4*>(g.res) + v);
     const uint32_t rv = __ldg(g.rev + v);
-    int32_t t = ldcg(g.term + v);
     if (h >= n || ex <= 0) return UNVIS;
+    // a node with residual to the sink has label 1: the seeds' label is never
+    // lowered, and a relabel of such a node gives 1 again
+    int32_t t = h == 1u ? ldcg(g.term + v) : 0;
     uint32_t next = UNVIS;
     const int nb[4] = {nb4.x, nb4.y, nb4.z, nb4.w};
     uint32_t r[4] = {r4.x, r4.y, r4.z, r4.w};
@@ -1165,8 +1304,9 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
     const uint32_t h0 = h;
     const int32_t t0 = t;
     long long pushed = 0;
+    unsigned long long self = 0;
     ++w.visits;
-    for (int step = 0; step < g.local_steps; ++step) {
+    for (int step = 0;; ++step) {
         if (t < 0 && h == 1u) {                       // v -> sink (.cu:220-236)
             const long long cap = -(long long)t;
             const long long d = ex < cap ? ex : cap;
@@ -1176,73 +1316,172 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
             w.sink += (unsigned long long)d;
             ++w.pushes;
         }
-        while (ex > 0) {                               // admissible pushes
-            int best = -1;
-            uint32_t bh = h;
+        // admissible pushes: the atomics of all slots are in flight together,
+        // and their results are read only once v's own update is too
+        unsigned long long o[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (nb[k] >= 0 && r[k] != 0u && hn[k] < bh) { bh = hn[k]; best = k; }
-            if (best < 0) break;
-            uint32_t rb = 0u;
-            int u = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k == best) { rb = r[k]; u = nb[k]; }
-            const uint32_t d = (uint32_t)(ex < (long long)rb ? ex : (long long)rb);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k == best) r[k] -= d;
+        for (int k = 0; k < 4; ++k) {
+            o[k] = 1ull;
+            if (nb[k] < 0 || r[k] == 0u || hn[k] >= h || ex <= 0) continue;
+            const uint32_t d = (uint32_t)(ex < (long long)r[k] ? ex : (long long)r[k]);
+            r[k] -= d;
             ex -= d;
             pushed += d;
-            const uint32_t rk = (rv >> (2 * best)) & 3u;
-            atomicSub(g.res + (size_t)v * 4u + best, d);
-            atomicAdd(g.res + (size_t)u * 4u + rk, d);
-            bool owner;
+            ++w.pushes;
+            const uint32_t rk = (rv >> (2 * k)) & 3u;
+            atomicSub(g.res + (size_t)v * 4u + k, d);
+            atomicAdd(g.res + (size_t)nb[k] * 4u + rk, d);
             if (kAgg) {
                 // lanes pushing to the same neighbour now add their amounts in
                 // one atomic, issued by the group's first lane, which takes
                 // ownership when the neighbour's excess was zero
                 const cg::coalesced_group active = cg::coalesced_threads();
-                const cg::coalesced_group same = cg::labeled_partition(active, (unsigned)u);
+                const cg::coalesced_group same = cg::labeled_partition(active, (unsigned)nb[k]);
                 const unsigned long long sum = cg::reduce(same, (unsigned long long)d,
                                                           cg::plus<unsigned long long>());
-                owner = same.thread_rank() == 0 &&
-                        atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + u), sum) == 0ull;
+                if (same.thread_rank() == 0)
+                    o[k] = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb[k]), sum);
             } else {
-                owner = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + u),
-                                  (unsigned long long)d) == 0ull;
+                o[k] = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb[k]),
+                                 (unsigned long long)d);
             }
-            if (owner) {
-                if (may_chain && next == UNVIS) next = (uint32_t)u;
-                else stage_push(g, st, (uint32_t)u);
-            }
-            ++w.pushes;
         }
-        if (ex <= 0) break;
-        uint32_t mh = (t < 0) ? 0u : UNVIS;            // relabel (.cu:274-301)
+        bool fin = ex <= 0;
+        if (!fin) {
+            uint32_t mh = (t < 0) ? 0u : UNVIS;        // relabel (.cu:274-301)
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (nb[k] >= 0 && r[k] != 0u && hn[k] < mh) mh = hn[k];
-        ++w.relabels;
-        if (mh == UNVIS) { h = UNVIS; break; }
-        h = mh + 1u;
-        if (h >= n) break;
+            for (int k = 0; k < 4; ++k)
+                if (nb[k] >= 0 && r[k] != 0u && hn[k] < mh) mh = hn[k];
+            ++w.relabels;
+            h = mh == UNVIS ? UNVIS : mh + 1u;
+            fin = h >= n || step + 1 >= g.local_steps;
+        }
+        if (fin) {
+            if (h != h0) g.height[v] = h;
+            if (t != t0) g.term[v] = t;
+            if (pushed)
+                self = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + v),
+                                 (unsigned long long)(-pushed));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (o[k] != 0ull) continue;   // not the push that took ownership
+            if (may_chain && next == UNVIS) next = (uint32_t)nb[k];
+            else stage_push(g, st, (uint32_t)nb[k]);
+        }
+        if (fin) break;
     }
-    if (h != h0) g.height[v] = h;
-    if (t != t0) g.term[v] = t;
-    long long now = ex;
-    if (pushed) {
-        const unsigned long long old = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + v),
-                                                 (unsigned long long)(-pushed));
-        now = (long long)old - pushed;
-    }
+    const long long now = pushed ? (long long)self - pushed : ex;
     if (now > 0 && h < n) stage_push(g, st, v);   // keeps ownership
     return next;
 }
 
-// One discharge round over cnt active nodes: discharge each, stage the nodes
-// that become (or stay) active, append them to the next active queue.
-// `first` is the thread's first entry (prefetch_entry).
+// discharge_node by four lanes, one per slot: the warp holds eight nodes,
+// `valid` where this lane's node exists; every lane of the warp calls it.
+__device__ __forceinline__ void discharge_quad(const SolveView& g, bool valid, uint32_t v, const Stage& st,
+                                               Work& w)
+{
+    const uint32_t n = g.n;
+    const uint32_t k = threadIdx.x & 3u;
+    uint32_t h = UNVIS, r = 0u, rv = 0u;
+    long long ex = 0;
+    int nb = -1;
+    int32_t t = 0;
+    if (valid) {
+        h = ldcg(g.height + v);
+        ex = ldcg(g.excess + v);
+        nb = __ldg(reinterpret_cast<const int*>(g.nbr) + (size_t)v * 4u + k);
+        r = ldcg(g.res + (size_t)v * 4u + k);
+        rv = __ldg(g.rev + v);
+    }
+    bool live = h < n && ex > 0;
+    uint32_t hn = UNVIS;
+    if (live && nb >= 0) hn = ldcg(g.height + nb);
+    if (h == 1u) t = ldcg(g.term + v);
+    if (nb < 0) r = 0u;
+    const bool lead = k == 0u;
+    if (live && lead) ++w.visits;
+    const uint32_t h0 = h;
+    const int32_t t0 = t;
+    long long pushed = 0;
+    unsigned long long o = 1ull, self = 0ull;
+    bool own = false;
+    for (int step = 0; __any_sync(0xffffffffu, live); ++step) {
+        if (live && t < 0 && h == 1u) {                // v -> sink (.cu:220-236)
+            const long long cap = -(long long)t;
+            const long long d = ex < cap ? ex : cap;
+            t = (int32_t)((long long)t + d);
+            ex -= d;
+            pushed += d;
+            if (lead) {
+                w.sink += (unsigned long long)d;
+                ++w.pushes;
+            }
+        }
+        // admissible slots take the excess (up to 2^32 - 1 of it a step) in
+        // slot order: saturating sums of the slots before this one
+        const uint32_t e = ex < 0xFFFFFFFFll ? (uint32_t)ex : 0xFFFFFFFFu;
+        const uint32_t a = (live && hn < h) ? r : 0u;
+        const uint32_t x1 = __shfl_xor_sync(0xffffffffu, a, 1);
+        const uint32_t p1 = a + x1 < a ? 0xFFFFFFFFu : a + x1;
+        const uint32_t x2 = __shfl_xor_sync(0xffffffffu, p1, 2);
+        const uint32_t total = p1 + x2 < p1 ? 0xFFFFFFFFu : p1 + x2;
+        const uint32_t b1 = (k & 1u) ? x1 : 0u, b2 = (k & 2u) ? x2 : 0u;
+        const uint32_t before = b1 + b2 < b1 ? 0xFFFFFFFFu : b1 + b2;
+        const uint32_t room = e > before ? e - before : 0u;
+        const uint32_t d = room < a ? room : a;
+        if (d) {
+            own = own || o == 0ull;   // an earlier step's push took ownership
+            o = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb), (unsigned long long)d);
+            r -= d;
+            ++w.pushes;
+        }
+        uint32_t mh = r ? hn : UNVIS;                  // relabel (.cu:274-301)
+        mh = min(mh, __shfl_xor_sync(0xffffffffu, mh, 1));
+        mh = min(mh, __shfl_xor_sync(0xffffffffu, mh, 2));
+        if (live) {
+            const uint32_t used = e < total ? e : total;
+            ex -= (long long)used;
+            pushed += (long long)used;
+            bool fin = ex <= 0;
+            if (!fin) {
+                if (t < 0) mh = 0u;
+                if (lead) ++w.relabels;
+                h = mh == UNVIS ? UNVIS : mh + 1u;
+                fin = h >= n || step + 1 >= g.local_steps;
+            }
+            if (fin) {
+                live = false;
+                self = (unsigned long long)ex;
+                if (lead) {
+                    if (pushed)
+                        self = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + v),
+                                         (unsigned long long)(-pushed));
+                    if (h != h0) g.height[v] = h;
+                    if (t != t0) g.term[v] = t;
+                }
+            }
+        }
+        // the residuals last: nothing waits for them, and the two excess
+        // updates above are on their way first
+        if (d) {
+            const uint32_t rk = (rv >> (2u * k)) & 3u;
+            atomicSub(g.res + (size_t)v * 4u + k, d);
+            atomicAdd(g.res + (size_t)nb * 4u + rk, d);
+        }
+    }
+    own = own || o == 0ull;
+    const bool keep = lead && valid && h < n && (long long)self - pushed > 0;   // keeps ownership
+    stage_push_warp(g, st, own, (uint32_t)nb, keep, v);
+}
+
+// One discharge round over cnt active nodes: discharge each, then up to
+// `levels` - 1 times the nodes the block staged in the level before (those that
+// became or stayed active; the block owns them), and append what the last
+// level left to the next active queue.  The stage is two halves of
+// stage_cap / 2 entries, ping-pong; entries that overflow a half go straight to
+// the queue.  With chains the round has one level.  `first` is the thread's
+// first entry (prefetch_entry).
 template <bool kAgg>
 __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t round, uint32_t cnt,
                                                uint32_t first, uint32_t* s_buf, uint32_t stage_cap,
@@ -1252,29 +1491,68 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
     const uint32_t* in = (round & 1) ? g.act[1] : g.act[0];
     uint32_t* out = (round & 1) ? g.act[0] : g.act[1];
     uint32_t* gcnt = &ctl->act_cnt[(round + 1) % 3];
-    const Stage st{s_buf, &s_m[0], stage_cap, gcnt, out};
-    const int hops = cnt <= g.chain_max_active ? g.chain_hops : 1;
-    for (uint32_t it = 0; it * (gridDim.x * DTPB) < cnt; ++it) {
-        const uint32_t i = queue_index(it, cnt);
-        if (i < cnt) {
-            uint32_t v = (it == 0 && cnt <= SPREAD_MAX) ? first : __ldcg(in + i);
-            if (v < g.n) {
-                for (int hop = 1;; ++hop) {
-                    v = discharge_node<kAgg>(g, v, st, hop < hops, w);
-                    if (v == UNVIS) break;
+    const bool narrow = cnt <= g.chain_max_active;
+    const int hops = narrow ? g.chain_hops : 1;
+    const int levels = narrow ? g.dis_levels : g.dis_levels_wide;
+    const uint32_t half = stage_cap / 2u;
+    const bool quads = !kAgg && hops <= 1 && levels > 1 && cnt <= SPREAD_MAX;
+    const uint32_t per_pass = gridDim.x * (quads ? DTPB / 4u : (uint32_t)DTPB);
+    for (uint32_t it = 0; it * per_pass < cnt; ++it) {
+        uint32_t* cur = s_buf;
+        uint32_t* nxt = s_buf + half;
+        const Stage st0{cur, &s_m[SUB], half, gcnt, out};
+        if (quads) {
+            const uint32_t i = quad_index(it);
+            const bool valid = i < cnt;
+            const uint32_t v = valid ? __ldcg(in + i) : 0u;
+            if (valid && v >= g.n) raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
+            if (__any_sync(0xffffffffu, valid)) discharge_quad(g, valid && v < g.n, v, st0, w);
+        } else {
+            const uint32_t i = queue_index(it, cnt);
+            if (i < cnt) {
+                uint32_t v = (it == 0 && cnt <= SPREAD_MAX) ? first : __ldcg(in + i);
+                if (v < g.n) {
+                    for (int hop = 1;; ++hop) {
+                        v = discharge_node<kAgg>(g, v, st0, hop < hops, w);
+                        if (v == UNVIS) break;
+                    }
+                } else {
+                    raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
                 }
-            } else {
-                raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
             }
         }
         __syncthreads();
+        uint32_t last = 0;   // ring slot of the last sub-level's count
+        for (int k = 1; k < levels; ++k) {
+            const uint32_t c = min(s_m[SUB + last], half);
+            if (c == 0u) break;
+            const uint32_t nx = last == 2u ? 0u : last + 1u;
+            // the slot after next was read before the last block barrier
+            if (threadIdx.x == 0) s_m[SUB + (nx == 2u ? 0u : nx + 1u)] = 0u;
+            const Stage st{nxt, &s_m[SUB + nx], half, gcnt, out};
+            if (!kAgg && c <= QUAD_MAX) {
+                // a warp without a node has nothing to do
+                for (uint32_t j0 = (threadIdx.x >> 5) * 8u; j0 < c; j0 += DTPB / 4u) {
+                    const uint32_t j = j0 + ((threadIdx.x & 31u) >> 2);
+                    const bool valid = j < c;
+                    discharge_quad(g, valid, valid ? cur[j] : 0u, st, w);
+                }
+            } else {
+                for (uint32_t j = threadIdx.x; j < c; j += DTPB) discharge_node<kAgg>(g, cur[j], st, false, w);
+            }
+            __syncthreads();
+            uint32_t* tmp = cur;
+            cur = nxt;
+            nxt = tmp;
+            last = nx;
+        }
         if (threadIdx.x == 0) {
-            s_m[2] = min(s_m[0], stage_cap);
-            s_m[0] = 0;
+            s_m[2] = min(s_m[SUB + last], half);
             s_m[4] = s_m[2] ? atomicAdd(gcnt, s_m[2]) : 0u;
         }
         __syncthreads();
-        flush_stage(s_buf, s_m[2], s_m[4], out, g.n, ctl);
+        flush_stage(cur, s_m[2], s_m[4], out, g.n, ctl);
+        if (threadIdx.x < 3) s_m[SUB + threadIdx.x] = 0u;
         __syncthreads();
     }
 }
@@ -1298,7 +1576,7 @@ __device__ __forceinline__ void reduce_work(Ctl* ctl, const Work& w, unsigned lo
 __global__ void __launch_bounds__(DTPB) k_discharge(SolveView g, uint32_t round)
 {
     __shared__ uint32_t s_buf[DTPB * 5];
-    __shared__ uint32_t s_m[8];
+    __shared__ uint32_t s_m[16];
     __shared__ unsigned long long s_red[DTPB / 32];
     Ctl* ctl = g.ctl;
     const uint32_t first = prefetch_entry((round & 1) ? g.act[1] : g.act[0], g.n);
@@ -1309,7 +1587,7 @@ __global__ void __launch_bounds__(DTPB) k_discharge(SolveView g, uint32_t round)
     }
     if (cnt == 0) return;
     Work w;
-    if (threadIdx.x == 0) s_m[0] = 0;
+    if (threadIdx.x < 16) s_m[threadIdx.x] = 0u;
     __syncthreads();
     discharge_body<false>(g, round, cnt, first, s_buf, DTPB * 5, s_m, w);
     reduce_work(ctl, w, 0ull, s_red);
@@ -1419,7 +1697,7 @@ template <bool kAgg, bool kTiles>
 __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, PersistParams p)
 {
     __shared__ __align__(16) uint32_t s_buf[DTPB * 8];   // 16-byte copies land here (tiles)
-    __shared__ uint32_t s_m[12];
+    __shared__ uint32_t s_m[16];
     __shared__ unsigned long long s_red[DTPB / 32];
     __shared__ int s_ok;
     Ctl* ctl = g.ctl;
@@ -1443,7 +1721,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
         tsm.low = tsm.am + RELABEL_TILE;
         tsm.list = reinterpret_cast<uint16_t*>(tsm.low + RELABEL_TILE);
     }
-    if (threadIdx.x < 12) s_m[threadIdx.x] = 0u;
+    if (threadIdx.x < 16) s_m[threadIdx.x] = 0u;
     // phase clock of block 0, read after each phase's closing barrier:
     // s_clk = {BFS, active sweep, discharge, last mark} (shared memory, so it
     // holds no registers through the solve)
@@ -1452,6 +1730,8 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
     __shared__ uint32_t s_step_cnt[3];
     __shared__ unsigned long long s_dr_ns[3], s_dr_t0;
     __shared__ uint32_t s_dr_cnt[3];
+    __shared__ unsigned long long s_rel_t0, s_dr_limit, s_win;
+    __shared__ uint32_t s_win_cnt;
     auto lap = [&](int phase) {
         if (lead) {
             const unsigned long long t = gtimer();
@@ -1484,6 +1764,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
         }
         while (ok) {
             // ---- global relabel (label-correcting steps, reachability exact) ----
+            if (lead) s_rel_t0 = gtimer();
             bfs_seed_body<false>(g, s_buf, s_buf + DTPB * 4, s_m, kTiles ? tstep + 1u : 0u);
             if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
             const uint32_t S0 = tstep + 1u;   // the seeds' tile step
@@ -1513,7 +1794,8 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
             bool exact = true;   // no chained step yet: every frontier node is labelled L
             uint32_t labelled = 0, bu_j = 0;
             for (; !kTiles;) {
-                const uint32_t first = prefetch_entry((L & 1) ? g.fr[1] : g.fr[0], g.n);
+                const uint32_t* fin = (L & 1) ? g.fr[1] : g.fr[0];
+                const uint32_t first = g.bfs_block_levels > 1 ? prefetch_quad(fin, g.n) : prefetch_entry(fin, g.n);
                 const uint32_t cnt = min(vload(&ctl->bfs_cnt[L % 3]), g.n);
                 if (cnt == 0) break;
                 if (lead) ctl->bfs_cnt[(L + 2) % 3] = 0u;
@@ -1556,7 +1838,8 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                     // expansions this step: the frontier, then per block and
                     // pass at most one stage half per sub-level
                     const unsigned long long nn = g.n;
-                    const unsigned long long passes = (cnt + gridDim.x * DTPB - 1u) / (gridDim.x * DTPB);
+                    const uint32_t per_pass = gridDim.x * (g.inm && cnt <= SPREAD_MAX ? DTPB / 4u : (uint32_t)DTPB);
+                    const unsigned long long passes = (cnt + per_pass - 1u) / per_pass;
                     const unsigned long long ex_max =
                         cnt + (unsigned long long)(g.bfs_block_levels - 1) * (DTPB * 4u) * gridDim.x * passes;
                     bfs_step_levels_body(g, L, cnt, first, s_buf, DTPB * 8, s_m, bfs_visits,
@@ -1591,6 +1874,11 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
             lap(0);
             active_sweep_body(g, s_buf, s_buf + DTPB * 4, s_m);
             if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+            if (lead) {
+                const unsigned long long t = gtimer();
+                s_win = (unsigned long long)(RELABEL_TIME_RATIO * (float)(t - s_rel_t0));
+                s_dr_limit = t + s_win;
+            }
             lap(1);
             if (vload(&ctl->act_cnt[0]) == 0u) break;   // maximum preflow
             if (g.nseg) retire_graphs(g);
@@ -1610,6 +1898,18 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                 if (lead) ctl->act_cnt[(r + 2) % 3] = 0u;
                 if (lead) s_dr_t0 = gtimer();   // shared: keeps the discharge's registers free
                 discharge_body<kAgg>(g, r, cnt, first, s_buf, DTPB * 8, s_m, w);
+                if (lead) {
+                    if (r == 0u) s_win_cnt = cnt;
+                    const unsigned long long t = gtimer();
+                    if (t > s_dr_limit) {
+                        if ((float)cnt * RELABEL_GAIN <= (float)s_win_cnt) {
+                            s_win_cnt = cnt;
+                            s_dr_limit = t + s_win;
+                        } else {
+                            ctl->stop_round = (uint32_t)rounds_total + 1u;
+                        }
+                    }
+                }
                 if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
                 if (lead) {
                     const int c = cnt <= 4096u ? 0 : (cnt <= 131072u ? 1 : 2);
@@ -1628,6 +1928,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                 }
                 if (p.relabel_rounds && r >= p.relabel_rounds) break;
                 if (budget && visits > budget) break;
+                if (vload(&ctl->stop_round) == (uint32_t)rounds_total) break;
             }
             if (!ok) break;
             if (lead) {
@@ -1879,14 +2180,16 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     GPUPR_CUDA(cudaMemsetAsync(g.ctl, 0, sizeof(Ctl), s));
     GPUPR_CUDA(cudaEventRecord(e0, s));
     SolveView gv = g;
-    // Chained discharge pays where a round is a latency chain (few active
-    // nodes) and can multiply node visits in wide rounds.  Measured on B200
-    // with 4 hops over 18 graphs below 1.5M free nodes: chaining in rounds of
-    // up to 131072 active nodes took 59.5 ms in all against 69.8 ms with
-    // 4096; between 1.5M and 2M, 32768 was best; above, only 4096 did not
-    // slow any graph down (a 2.9M-node torus: 6.6 ms, 10.0 with 32768).  The
-    // autotuner may pick another setting.
-    gv.chain_hops = opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : 4;
+    // Discharge rounds run in block sub-levels; chains (a thread going on from
+    // node to node) are an option and replace the sub-levels of the rounds
+    // they apply to.  A caller's small round limit counts rounds of one
+    // discharge per queued node, so it turns the sub-levels off (a sub-level
+    // round does the work of many; 16384 is far above the rounds any of the
+    // graphs measured needs, at most 3,200 single ones).
+    const bool plain_rounds = opt.max_rounds < 16384ull;
+    gv.chain_hops = opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : plain_rounds ? 4 : 1;
+    gv.dis_levels = plain_rounds ? 1 : gv.chain_hops > 1 ? 1 : DIS_LEVELS;
+    gv.dis_levels_wide = plain_rounds ? 1 : DIS_LEVELS_WIDE;
     gv.bfs_hops = opt.bfs_chain_hops > 0 ? std::min(opt.bfs_chain_hops, 64) : BFS_CHAIN_HOPS;
     // BFS steps expand BFS_BLOCK_LEVELS levels per block by default (measured
     // against per-thread chains of 4: benchmark graph 77.7 -> 68.0 ms, 8M-tet
@@ -1906,9 +2209,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
                                          : BFS_TAIL_DEFAULT;
     gv.chain_max_active = opt.chain_max_active > 0 ? (uint32_t)opt.chain_max_active
                           : tuned                  ? (uint32_t)te.chain_max_active
-                          : g.n < 1500000u         ? 131072u
-                          : g.n < 2000000u         ? 32768u
-                                                   : 4096u;
+                                                   : DIS_NARROW_MAX;
     void* args[] = {&gv, &p};
     GPUPR_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(DTPB), args, dsmem, s));
     GPUPR_CUDA(cudaEventRecord(e1, s));
