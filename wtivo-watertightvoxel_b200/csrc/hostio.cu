@@ -3,11 +3,16 @@
 // The drop-in boundary takes numpy arrays (vertices, labels in; labels out),
 // and the serving loop takes whole graphs from host memory.  A plain
 // cudaMemcpyAsync from pageable memory goes through the driver's own staging
-// at the speed of one host thread.  Here each copy is cut into chunks that
-// rotate through a few pinned staging buffers: a small pool of host threads
-// copies chunk c+1 between the caller's array and a staging buffer while the
-// DMA engine moves chunk c, so the copy runs near the PCIe rate instead of
-// one core's memcpy rate.  Pinned source/destination arrays skip the staging.
+// at the speed of one host thread.  Here a copy is cut into 1 MiB pieces that
+// rotate through a ring of pinned buffers: the calling thread and a small pool
+// of host threads each take the next piece, copy it between the caller's
+// array and its buffer and issue its DMA, so host copies and DMA overlap and the
+// copy runs near the PCIe rate.  The threads are woken once per copy, one waking
+// the next, and the caller starts at once: waking all of them for every 8 MiB
+// chunk, and waiting for the slowest of them at its end, cost more than the
+// copy itself up to tens of MB (13 MB: 1.63 -> 0.6-0.8 ms, 34 MB: 1.82 -> 1.4-1.6, the
+// driver's own path 0.67 and 1.74; 102 MB 3.6 -> 3.4-3.9).  Pinned
+// source/destination arrays skip the staging.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -16,10 +21,12 @@
 #include <condition_variable>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -28,14 +35,14 @@
 namespace gpupr {
 namespace {
 
-constexpr size_t kChunk = 8u << 20;     // bytes per staging buffer
-constexpr int kSlots = 4;               // staging buffers per direction and device
+constexpr size_t kPiece = 1u << 20;     // bytes per staging buffer
+constexpr int kSlots = 32;              // staging buffers per set
 constexpr size_t kDirect = 1u << 20;    // below this, the driver's own path
 
-// A fixed set of host worker threads that run the parts of one job (a
-// memcpy or a row gather) in parallel; the calling thread takes parts too.
-// Each job is its own object that workers pick up under the pool mutex, so a
-// worker can never take a part of a later job by mistake.
+// A fixed set of host worker threads that run the parts of one job in
+// parallel; the calling thread takes parts too.  Each job is its own object
+// that workers pick up under the pool mutex, so a worker can never take a part
+// of a later job by mistake.
 class CopyPool {
 public:
     CopyPool()
@@ -56,56 +63,47 @@ public:
         cv_.notify_all();
         for (auto& t : workers_) t.join();
     }
-    int threads() const { return (int)workers_.size() + 1; }
 
-    // Runs fn(0..parts-1), returns when every part is done.
-    void run(int parts, std::function<void(int)> fn)
+    // Runs fn(0..parts-1), each part once and in ascending order of start, on
+    // the calling thread and up to `helpers` workers; returns when every part is
+    // done.
+    void run(int64_t parts, int64_t helpers, const std::function<void(int64_t)>& fn)
     {
-        if (parts <= 1 || workers_.empty()) {
-            for (int p = 0; p < parts; ++p) fn(p);
+        const int64_t calls = std::min(std::min((int64_t)workers_.size(), helpers), parts - 1);
+        if (calls <= 0) {
+            for (int64_t p = 0; p < parts; ++p) fn(p);
             return;
         }
         auto job = std::make_shared<Job>();
-        job->fn = std::move(fn);
+        job->fn = &fn;
         job->parts = parts;
         job->left = parts;
-        {
+        try {
             std::lock_guard<std::mutex> lk(mu_);
-            job_ = job;
-            ++gen_;
+            for (int64_t i = 0; i < calls; ++i) calls_.push_back(job);
+        } catch (const std::bad_alloc&) {
+            // fewer helpers; the job must not be left to those it has by unwinding
         }
-        cv_.notify_all();
+        cv_.notify_one();   // that thread wakes the next
         job->run();
         std::unique_lock<std::mutex> lk(job->mu);
         job->cv.wait(lk, [&] { return job->left == 0; });
     }
 
-    void copy(void* dst, const void* src, size_t n)
-    {
-        const int parts = (int)std::min<size_t>(threads(), std::max<size_t>(1, n / (1u << 20)));
-        const size_t per = (n + parts - 1) / parts;
-        char* d = static_cast<char*>(dst);
-        const char* s = static_cast<const char*>(src);
-        run(parts, [=](int p) {
-            const size_t b = (size_t)p * per, e = std::min(n, b + per);
-            if (b < e) std::memcpy(d + b, s + b, e - b);
-        });
-    }
-
 private:
     struct Job {
-        std::function<void(int)> fn;
-        int parts = 0;
-        std::atomic<int> next{0};
-        int left = 0;
+        const std::function<void(int64_t)>* fn = nullptr;   // alive while parts are left
+        int64_t parts = 0;
+        std::atomic<int64_t> next{0};
+        int64_t left = 0;
         std::mutex mu;
         std::condition_variable cv;
         void run()
         {
             for (;;) {
-                const int p = next.fetch_add(1);
+                const int64_t p = next.fetch_add(1);
                 if (p >= parts) return;
-                fn(p);
+                (*fn)(p);
                 std::lock_guard<std::mutex> lk(mu);
                 if (--left == 0) cv.notify_all();
             }
@@ -113,25 +111,26 @@ private:
     };
     void work()
     {
-        uint64_t seen = 0;
         for (;;) {
             std::shared_ptr<Job> job;
+            bool more;
             {
                 std::unique_lock<std::mutex> lk(mu_);
-                cv_.wait(lk, [&] { return stop_ || gen_ != seen; });
+                cv_.wait(lk, [&] { return stop_ || !calls_.empty(); });
                 if (stop_) return;
-                seen = gen_;
-                job = job_;
+                job = std::move(calls_.front());
+                calls_.pop_front();
+                more = !calls_.empty();
             }
-            if (job) job->run();
+            if (more) cv_.notify_one();
+            job->run();
         }
     }
 
     std::vector<std::thread> workers_;
     std::mutex mu_;
     std::condition_variable cv_;
-    std::shared_ptr<Job> job_;
-    uint64_t gen_ = 0;
+    std::deque<std::shared_ptr<Job>> calls_;   // one entry per thread a job may use
     bool stop_ = false;
 };
 
@@ -146,14 +145,13 @@ struct Staging {
     char* pin = nullptr;
     cudaEvent_t ev[kSlots] = {};
     bool pending[kSlots] = {};
-    bool ok = false;
 };
 
 // Staging sets per device and direction (0 = to device, 1 = to host) that
 // host threads can hold at the same time, so that copies issued by
 // different threads (the server's two lanes, each uploading its own batch)
 // run side by side instead of queueing on one set; each set is kSlots x
-// kChunk pinned bytes, made on first use with its device current.
+// kPiece pinned bytes, made on first use with its device current.
 constexpr int kSets = 3;
 
 // A staging set held by one copy until the lease goes out of scope.
@@ -181,10 +179,9 @@ StagingLease staging(int dir)
         }
         if ((int)sets.size() < kSets) {
             auto s = std::make_unique<Staging>();
-            GPUPR_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->pin), kChunk * kSlots, cudaHostAllocPortable));
+            GPUPR_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->pin), kPiece * kSlots, cudaHostAllocPortable));
             for (int i = 0; i < kSlots; ++i)
                 GPUPR_CUDA(cudaEventCreateWithFlags(&s->ev[i], cudaEventDisableTiming));
-            s->ok = true;
             std::unique_lock<std::mutex> l(s->mu);
             Staging* p = s.get();
             sets.push_back(std::move(s));
@@ -216,6 +213,47 @@ bool is_pinned(const void* p)
     return a.type == cudaMemoryTypeHost;
 }
 
+// Host threads that help the caller with a memcpy through the staging: waking a
+// sleeping thread costs about what copying 1 MiB does, so each has to bring
+// several pieces' worth.  Measured with 0 / 1 / 2 / 3 / 6 helpers: 8 MB 0.62 / 0.36
+// / 0.33 / 0.34 / 0.99 ms, 13 MB 1.0 / 0.56 / 0.75 / 0.91 / 1.19, 34 MB 3.4 / 1.75 /
+// 1.66 / 1.28 / 1.97, 102 MB 11.9 / 6.2 / 4.5 / 3.8 / 3.4.
+int64_t copy_helpers(size_t bytes)
+{
+    return bytes < (4u << 20) ? 0 : std::max<int64_t>(1, (int64_t)(bytes / (10u << 20)));
+}
+
+// Runs `pieces` pieces through a staging set, each by one host thread (the
+// caller's device current): piece p uses buffer p % kSlots, after piece p -
+// kSlots is through with it.  step(p, pin, ev) copies piece p and issues its
+// DMA.  The first CUDA error is thrown by the caller's thread once all pieces
+// have been taken.
+template <class Step>
+void run_pieces(Staging& st, int64_t pieces, int64_t helpers, const Step& step)
+{
+    int dev = 0;
+    GPUPR_CUDA(cudaGetDevice(&dev));
+    std::atomic<int64_t> done[kSlots];   // pieces a buffer has served
+    for (auto& d : done) d.store(0, std::memory_order_relaxed);
+    std::atomic<int> err{(int)cudaSuccess};
+    copy_pool().run(pieces, helpers, [&](int64_t p) {
+        const int k = (int)(p % kSlots);
+        // pieces start in order, so an earlier one of this buffer is on its way
+        while (done[k].load(std::memory_order_acquire) != p / kSlots) std::this_thread::yield();
+        if (err.load(std::memory_order_relaxed) == (int)cudaSuccess) {
+            cudaError_t e = cudaSetDevice(dev);
+            if (e == cudaSuccess && st.pending[k]) {
+                e = cudaEventSynchronize(st.ev[k]);
+                if (e == cudaSuccess) st.pending[k] = false;
+            }
+            if (e == cudaSuccess) e = step(p, st.pin + (size_t)k * kPiece, k);
+            if (e != cudaSuccess) err.store((int)e, std::memory_order_relaxed);
+        }
+        done[k].fetch_add(1, std::memory_order_release);
+    });
+    GPUPR_CUDA((cudaError_t)err.load());
+}
+
 }  // namespace
 
 void host_to_device(void* d_dst, const void* h_src, size_t bytes, cudaStream_t s)
@@ -227,20 +265,16 @@ void host_to_device(void* d_dst, const void* h_src, size_t bytes, cudaStream_t s
     }
     StagingLease lease = staging(0);
     Staging& st = *lease.st;
-    settle(st);
     const char* src = static_cast<const char*>(h_src);
     char* dst = static_cast<char*>(d_dst);
-    const size_t nch = (bytes + kChunk - 1) / kChunk;
-    for (size_t c = 0; c < nch; ++c) {
-        const int k = (int)(c % kSlots);
-        const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
-        char* pin = st.pin + (size_t)k * kChunk;
-        if (st.pending[k]) GPUPR_CUDA(cudaEventSynchronize(st.ev[k]));
-        copy_pool().copy(pin, src + off, len);
-        GPUPR_CUDA(cudaMemcpyAsync(dst + off, pin, len, cudaMemcpyHostToDevice, s));
-        GPUPR_CUDA(cudaEventRecord(st.ev[k], s));
+    run_pieces(st, (int64_t)((bytes + kPiece - 1) / kPiece), copy_helpers(bytes), [&](int64_t p, char* pin, int k) {
+        const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
+        std::memcpy(pin, src + off, len);
+        const cudaError_t e = cudaMemcpyAsync(dst + off, pin, len, cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) return e;
         st.pending[k] = true;
-    }
+        return cudaEventRecord(st.ev[k], s);
+    });
 }
 
 void device_to_host(void* h_dst, const void* d_src, size_t bytes, cudaStream_t s)
@@ -256,30 +290,30 @@ void device_to_host(void* h_dst, const void* d_src, size_t bytes, cudaStream_t s
     settle(st);
     const char* src = static_cast<const char*>(d_src);
     char* dst = static_cast<char*>(h_dst);
-    const size_t nch = (bytes + kChunk - 1) / kChunk;
-    auto issue = [&](size_t c) {
-        const int k = (int)(c % kSlots);
-        const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
-        GPUPR_CUDA(cudaMemcpyAsync(st.pin + (size_t)k * kChunk, src + off, len,
-                                   cudaMemcpyDeviceToHost, s));
-        GPUPR_CUDA(cudaEventRecord(st.ev[k], s));
+    const int64_t pieces = (int64_t)((bytes + kPiece - 1) / kPiece);
+    auto issue = [&](int64_t p) {
+        const int k = (int)(p % kSlots);
+        const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
+        const cudaError_t e = cudaMemcpyAsync(st.pin + (size_t)k * kPiece, src + off, len,
+                                              cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) return e;
         st.pending[k] = true;
+        return cudaEventRecord(st.ev[k], s);
     };
-    for (size_t c = 0; c < std::min<size_t>(nch, kSlots); ++c) issue(c);
-    for (size_t c = 0; c < nch; ++c) {
-        const int k = (int)(c % kSlots);
-        const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
-        GPUPR_CUDA(cudaEventSynchronize(st.ev[k]));
-        copy_pool().copy(dst + off, st.pin + (size_t)k * kChunk, len);
-        st.pending[k] = false;
-        if (c + kSlots < nch) issue(c + kSlots);
-    }
+    // a ring of DMAs ahead; a piece's thread waits for it (run_pieces), copies
+    // it out and issues the one that follows in its buffer
+    for (int64_t p = 0; p < std::min<int64_t>(pieces, kSlots); ++p) GPUPR_CUDA(issue(p));
+    run_pieces(st, pieces, copy_helpers(bytes), [&](int64_t p, char* pin, int) {
+        const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
+        std::memcpy(dst + off, pin, len);
+        return p + kSlots < pieces ? issue(p + kSlots) : cudaSuccess;
+    });
 }
 
 // Nx4 integer topology (int32 or int64 elements, any byte strides, e.g. a
 // Fortran-ordered matrix) -> contiguous int32 Nx4 on the device.  Rows are
-// gathered chunk by chunk into the pinned staging by the host pool while the
-// previous chunk is in flight; int64 values are narrowed the way numpy's
+// gathered piece by piece into the pinned staging by the host threads while
+// earlier pieces are in flight; int64 values are narrowed the way numpy's
 // astype(int32) narrows them (low 32 bits).
 void upload_topology(int32_t* d_out, const void* host, uint64_t rows, int64_t row_stride,
                      int64_t col_stride, int elem_bytes, cudaStream_t s)
@@ -292,38 +326,31 @@ void upload_topology(int32_t* d_out, const void* host, uint64_t rows, int64_t ro
     const char* base = static_cast<const char*>(host);
     StagingLease lease = staging(0);
     Staging& st = *lease.st;
-    settle(st);
-    const uint64_t per_chunk = kChunk / 16u;
-    const uint64_t nch = (rows + per_chunk - 1) / per_chunk;
-    CopyPool& pool = copy_pool();
-    for (uint64_t c = 0; c < nch; ++c) {
-        const int k = (int)(c % kSlots);
-        const uint64_t r0 = c * per_chunk, r1 = std::min(rows, r0 + per_chunk);
-        int32_t* pin = reinterpret_cast<int32_t*>(st.pin + (size_t)k * kChunk);
-        if (st.pending[k]) GPUPR_CUDA(cudaEventSynchronize(st.ev[k]));
-        const int parts = std::max(1, std::min(pool.threads(), (int)((r1 - r0) / 16384u)));
-        const uint64_t per = (r1 - r0 + parts - 1) / parts;
-        pool.run(parts, [=](int p) {
-            const uint64_t a = r0 + (uint64_t)p * per, z = std::min(r1, a + per);
-            for (uint64_t r = a; r < z; ++r) {
-                const char* row = base + (int64_t)r * row_stride;
-                int32_t* o = pin + (r - r0) * 4u;
-                for (int j = 0; j < 4; ++j) {
-                    const char* e = row + (int64_t)j * col_stride;
-                    if (elem_bytes == 8) {
-                        int64_t v;
-                        std::memcpy(&v, e, 8);
-                        o[j] = (int32_t)(uint32_t)(uint64_t)v;
-                    } else {
-                        std::memcpy(&o[j], e, 4);
-                    }
+    const uint64_t per = kPiece / 16u;
+    // a strided gather costs several times a memcpy: a helper per piece
+    const int64_t pieces = (int64_t)((rows + per - 1) / per);
+    run_pieces(st, pieces, pieces, [&](int64_t p, char* pin, int k) {
+        const uint64_t r0 = (uint64_t)p * per, r1 = std::min(rows, r0 + per);
+        int32_t* out = reinterpret_cast<int32_t*>(pin);
+        for (uint64_t r = r0; r < r1; ++r) {
+            const char* row = base + (int64_t)r * row_stride;
+            int32_t* o = out + (r - r0) * 4u;
+            for (int j = 0; j < 4; ++j) {
+                const char* e = row + (int64_t)j * col_stride;
+                if (elem_bytes == 8) {
+                    int64_t v;
+                    std::memcpy(&v, e, 8);
+                    o[j] = (int32_t)(uint32_t)(uint64_t)v;
+                } else {
+                    std::memcpy(&o[j], e, 4);
                 }
             }
-        });
-        GPUPR_CUDA(cudaMemcpyAsync(d_out + r0 * 4u, pin, (r1 - r0) * 16u, cudaMemcpyHostToDevice, s));
-        GPUPR_CUDA(cudaEventRecord(st.ev[k], s));
+        }
+        const cudaError_t e = cudaMemcpyAsync(d_out + r0 * 4u, pin, (r1 - r0) * 16u, cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) return e;
         st.pending[k] = true;
-    }
+        return cudaEventRecord(st.ev[k], s);
+    });
 }
 
 namespace {
