@@ -1316,12 +1316,16 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
             w.sink += (unsigned long long)d;
             ++w.pushes;
         }
-        // admissible pushes: the atomics of all slots are in flight together,
-        // and their results are read only once v's own update is too
+        // admissible pushes: the atomics of all slots are in flight together.
+        // v's own residuals return before v's excess is released below: the
+        // node is another thread's the moment its excess is 0, and that
+        // thread must not read a residual that is still to be lowered.
         unsigned long long o[4];
+        uint32_t left[4];   // v's residuals as the pushes found them
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             o[k] = 1ull;
+            left[k] = 0xFFFFFFFFu;
             if (nb[k] < 0 || r[k] == 0u || hn[k] >= h || ex <= 0) continue;
             const uint32_t d = (uint32_t)(ex < (long long)r[k] ? ex : (long long)r[k]);
             r[k] -= d;
@@ -1329,7 +1333,7 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
             pushed += d;
             ++w.pushes;
             const uint32_t rk = (rv >> (2 * k)) & 3u;
-            atomicSub(g.res + (size_t)v * 4u + k, d);
+            left[k] = atomicSub(g.res + (size_t)v * 4u + k, d);
             atomicAdd(g.res + (size_t)nb[k] * 4u + rk, d);
             if (kAgg) {
                 // lanes pushing to the same neighbour now add their amounts in
@@ -1346,6 +1350,9 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
                                  (unsigned long long)d);
             }
         }
+        // others only ever raise v's residuals meanwhile
+        if (left[0] < r[0] || left[1] < r[1] || left[2] < r[2] || left[3] < r[3])
+            raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
         bool fin = ex <= 0;
         if (!fin) {
             uint32_t mh = (t < 0) ? 0u : UNVIS;        // relabel (.cu:274-301)
@@ -1358,7 +1365,10 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
         }
         if (fin) {
             if (h != h0) g.height[v] = h;
-            if (t != t0) g.term[v] = t;
+            if (t != t0) {
+                g.term[v] = t;
+                __threadfence();   // the next owner reads it
+            }
             if (pushed)
                 self = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + v),
                                  (unsigned long long)(-pushed));
@@ -1377,16 +1387,23 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
 }
 
 // discharge_node by four lanes, one per slot: the warp holds eight nodes,
-// `valid` where this lane's node exists; every lane of the warp calls it.
+// `valid` where this lane's node exists; every lane of the warp calls it.  On a
+// short list a sub-level is one chain of memory round trips (the node's state,
+// its neighbours' heights, the pushes, the release of its excess) and of the
+// instructions between them: about 2.2 us from node to node on a path graph,
+// 1,500 cycles of it the push and the load that depends on it.  Going on with the
+// pushed-to node in the same lanes, its state loaded during the push, took 2.0 us
+// there, but excess then runs ahead of what it should merge with (8 nodes in a
+// row: a 200k-node integer graph 1.6 -> 2.7 ms, an 8M-tet open box 18.6 -> 26.7).
 __device__ __forceinline__ void discharge_quad(const SolveView& g, bool valid, uint32_t v, const Stage& st,
                                                Work& w)
 {
     const uint32_t n = g.n;
     const uint32_t k = threadIdx.x & 3u;
-    uint32_t h = UNVIS, r = 0u, rv = 0u;
+    const bool lead = k == 0u;
+    uint32_t h = UNVIS, r = 0u, rv = 0u, hn = UNVIS;
     long long ex = 0;
     int nb = -1;
-    int32_t t = 0;
     if (valid) {
         h = ldcg(g.height + v);
         ex = ldcg(g.excess + v);
@@ -1395,26 +1412,27 @@ __device__ __forceinline__ void discharge_quad(const SolveView& g, bool valid, u
         rv = __ldg(g.rev + v);
     }
     bool live = h < n && ex > 0;
-    uint32_t hn = UNVIS;
     if (live && nb >= 0) hn = ldcg(g.height + nb);
-    if (h == 1u) t = ldcg(g.term + v);
+    int32_t t = 0;
+    if (live && h == 1u) t = ldcg(g.term + v);
     if (nb < 0) r = 0u;
-    const bool lead = k == 0u;
     if (live && lead) ++w.visits;
     const uint32_t h0 = h;
     const int32_t t0 = t;
+    const bool mine = live;
     long long pushed = 0;
-    unsigned long long o = 1ull, self = 0ull;
+    unsigned long long o = 1ull;
+    uint32_t left = 0u, d = 0u;
     bool own = false;
     for (int step = 0; __any_sync(0xffffffffu, live); ++step) {
         if (live && t < 0 && h == 1u) {                // v -> sink (.cu:220-236)
             const long long cap = -(long long)t;
-            const long long d = ex < cap ? ex : cap;
-            t = (int32_t)((long long)t + d);
-            ex -= d;
-            pushed += d;
+            const long long x = ex < cap ? ex : cap;
+            t = (int32_t)((long long)t + x);
+            ex -= x;
+            pushed += x;
             if (lead) {
-                w.sink += (unsigned long long)d;
+                w.sink += (unsigned long long)x;
                 ++w.pushes;
             }
         }
@@ -1429,49 +1447,54 @@ __device__ __forceinline__ void discharge_quad(const SolveView& g, bool valid, u
         const uint32_t b1 = (k & 1u) ? x1 : 0u, b2 = (k & 2u) ? x2 : 0u;
         const uint32_t before = b1 + b2 < b1 ? 0xFFFFFFFFu : b1 + b2;
         const uint32_t room = e > before ? e - before : 0u;
-        const uint32_t d = room < a ? room : a;
-        if (d) {
-            own = own || o == 0ull;   // an earlier step's push took ownership
+        const uint32_t y = room < a ? room : a;
+        if (y) {
+            if (d) {   // pushed in an earlier step too: look at that push now
+                own = own || o == 0ull;
+                if (left < d) raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+            }
+            d = y;
+            const uint32_t rk = (rv >> (2u * k)) & 3u;
             o = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb), (unsigned long long)d);
+            left = atomicSub(g.res + (size_t)v * 4u + k, d);
+            atomicAdd(g.res + (size_t)nb * 4u + rk, d);
             r -= d;
             ++w.pushes;
         }
-        uint32_t mh = r ? hn : UNVIS;                  // relabel (.cu:274-301)
-        mh = min(mh, __shfl_xor_sync(0xffffffffu, mh, 1));
-        mh = min(mh, __shfl_xor_sync(0xffffffffu, mh, 2));
         if (live) {
             const uint32_t used = e < total ? e : total;
             ex -= (long long)used;
             pushed += (long long)used;
-            bool fin = ex <= 0;
-            if (!fin) {
+        }
+        live = live && ex > 0;
+        if (__any_sync(0xffffffffu, live)) {
+            uint32_t mh = r ? hn : UNVIS;              // relabel (.cu:274-301)
+            mh = min(mh, __shfl_xor_sync(0xffffffffu, mh, 1));
+            mh = min(mh, __shfl_xor_sync(0xffffffffu, mh, 2));
+            if (live) {
                 if (t < 0) mh = 0u;
                 if (lead) ++w.relabels;
                 h = mh == UNVIS ? UNVIS : mh + 1u;
-                fin = h >= n || step + 1 >= g.local_steps;
+                live = h < n && step + 1 < g.local_steps;
             }
-            if (fin) {
-                live = false;
-                self = (unsigned long long)ex;
-                if (lead) {
-                    if (pushed)
-                        self = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + v),
-                                         (unsigned long long)(-pushed));
-                    if (h != h0) g.height[v] = h;
-                    if (t != t0) g.term[v] = t;
-                }
-            }
-        }
-        // the residuals last: nothing waits for them, and the two excess
-        // updates above are on their way first
-        if (d) {
-            const uint32_t rk = (rv >> (2u * k)) & 3u;
-            atomicSub(g.res + (size_t)v * 4u + k, d);
-            atomicAdd(g.res + (size_t)nb * 4u + rk, d);
         }
     }
+    // release v's excess once all four lanes know v's residuals lowered
+    // (discharge_node): the checks wait for every lane's atomic
+    if (d && left < d) raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+    __syncwarp();
+    unsigned long long self = (unsigned long long)ex;
+    if (mine && lead) {
+        if (h != h0) g.height[v] = h;
+        if (t != t0) {
+            g.term[v] = t;
+            __threadfence();   // the next owner reads it
+        }
+        if (pushed)
+            self = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + v), (unsigned long long)(-pushed));
+    }
     own = own || o == 0ull;
-    const bool keep = lead && valid && h < n && (long long)self - pushed > 0;   // keeps ownership
+    const bool keep = mine && lead && h < n && (long long)self - pushed > 0;   // keeps ownership
     stage_push_warp(g, st, own, (uint32_t)nb, keep, v);
 }
 
