@@ -320,6 +320,7 @@ __device__ __forceinline__ uint32_t queue_index(uint32_t it, uint32_t cnt)
 // 26.6 -> 18.6 ms with the same schedule).  Above three passes of 64 nodes the
 // threads are better spent on more nodes at a time.
 constexpr uint32_t QUAD_MAX = 192u;
+constexpr uint32_t BFS_QUAD_MAX = 96u;
 
 // Queue index of a thread's node in pass `it` when four lanes share a node:
 // eight entries per warp, dealt round-robin over the blocks.
@@ -947,6 +948,14 @@ __device__ __forceinline__ void bfs_expand_one(const SolveView& g, uint32_t u, u
     }
 }
 
+// Atomics under a predicate, without a branch: where a list is short a warp
+// runs alone, and every branch that may diverge costs it tens of cycles to
+// resolve and to reconverge.  x keeps its value where p does not hold.
+__device__ __forceinline__ void atom_min_if(bool p, uint32_t& x, uint32_t* a, uint32_t v)
+{
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %1, 0; @q atom.global.min.u32 %0, [%2], %3; }"
+                 : "+r"(x) : "r"((unsigned)p), "l"(a), "r"(v) : "memory");
+}
 // Appends this lane's entries to the stage: u where `want` holds, v where
 // `want2` does; every lane of the warp calls it: one shared atomic per warp.
 __device__ __forceinline__ void stage_push_warp(const SolveView& g, const Stage& st, bool want, uint32_t u,
@@ -954,55 +963,49 @@ __device__ __forceinline__ void stage_push_warp(const SolveView& g, const Stage&
 {
     const unsigned b1 = __ballot_sync(0xffffffffu, want);
     const unsigned b2 = __ballot_sync(0xffffffffu, want2);
-    if (!(b1 | b2)) return;
+    const uint32_t c1 = (uint32_t)__popc(b1), total = c1 + (uint32_t)__popc(b2);
+    if (total == 0u) return;
     const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     uint32_t base = 0;
-    if (lane == 0u) base = atomicAdd(st.cnt, (uint32_t)(__popc(b1) + __popc(b2)));
+    if (lane == 0u) base = atomicAdd(st.cnt, total);
     base = __shfl_sync(0xffffffffu, base, 0);
-    uint32_t idx = base + (uint32_t)__popc(b1 & below);
-    if (want) {
-        if (idx < st.cap) {
-            st.buf[idx] = u;
-        } else {
-            const uint32_t pos = atomicAdd(st.gcnt, 1u);
-            if (pos < g.n) st.out[pos] = u;
-            else raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
-        }
+    const uint32_t i1 = base + (uint32_t)__popc(b1 & below);
+    const uint32_t i2 = base + c1 + (uint32_t)__popc(b2 & below);
+    if (base + total <= st.cap) {
+        if (want) st.buf[i1] = u;
+        if (want2) st.buf[i2] = v;
+        return;
     }
-    if (want2) {
-        idx = base + (uint32_t)(__popc(b1) + __popc(b2 & below));
+    auto put = [&](uint32_t idx, uint32_t x) {   // past the stage: into the queue
         if (idx < st.cap) {
-            st.buf[idx] = v;
-        } else {
-            const uint32_t pos = atomicAdd(st.gcnt, 1u);
-            if (pos < g.n) st.out[pos] = v;
-            else raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+            st.buf[idx] = x;
+            return;
         }
-    }
+        const uint32_t pos = atomicAdd(st.gcnt, 1u);
+        if (pos < g.n) st.out[pos] = x;
+        else raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+    };
+    if (want) put(i1, u);
+    if (want2) put(i2, v);
 }
 
-// bfs_expand_one by four lanes, one per slot (in-arc masks only): the warp
-// holds eight nodes, `valid` where this lane's node exists.
-__device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, uint32_t u, uint32_t L,
-                                                bool exact, const Stage& st, bool propagate,
-                                                unsigned long long& visits, uint32_t* s_m)
+// bfs_expand_one by four lanes, one per slot (in-arc masks, top-down only): the
+// warp holds eight nodes, `valid` where this lane's node exists.
+__device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, uint32_t u, const Stage& st,
+                                                bool propagate, unsigned long long& visits)
 {
     const uint32_t k = threadIdx.x & 3u;
-    bool want = false;
-    int nb = 0;
-    if (valid) {
-        const uint32_t hu = exact ? L : ldcg(g.height + u);
-        nb = __ldg(reinterpret_cast<const int*>(g.nbr) + (size_t)u * 4u + k);
-        const uint32_t m = __ldcg(g.inm + u);
-        if (k == 0u) ++visits;
-        const uint32_t cand = hu + 1u;
-        if (((m >> k) & 1u) && ldcg(g.height + nb) > cand) {
-            const uint32_t old = atomicMin(g.height + nb, cand);
-            if (g.bottom_up && old == UNVIS) atomicAdd(&s_m[6], 1u);   // a first label
-            want = old > cand && (old == UNVIS || propagate);
-        }
-    }
-    stage_push_warp(g, st, want, (uint32_t)nb);
+    u = valid ? u : 0u;   // lanes without a node read node 0 and do nothing with it
+    const uint32_t cand = ldcg(g.height + u) + 1u;
+    const int nb = __ldg(reinterpret_cast<const int*>(g.nbr) + (size_t)u * 4u + k);
+    const uint32_t m = __ldcg(g.inm + u);
+    const bool arc = valid && ((m >> k) & 1u);
+    const uint32_t v = arc ? (uint32_t)nb : u;
+    const bool lower = arc && ldcg(g.height + v) > cand;
+    uint32_t old = 0u;
+    atom_min_if(lower, old, g.height + v, cand);
+    visits += (valid && k == 0u) ? 1ull : 0ull;
+    stage_push_warp(g, st, lower && old > cand && (old == UNVIS || propagate), v);
 }
 
 // A BFS step of the persistent engine with block sub-levels (option
@@ -1026,7 +1029,8 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
     uint32_t* out = (L & 1) ? g.fr[0] : g.fr[1];
     uint32_t* gcnt = &ctl->bfs_cnt[(L + 1) % 3];
     const uint32_t half = stage_cap / 2u;
-    const bool quads = g.inm && cnt <= SPREAD_MAX;
+    const bool may_quad = g.inm && !g.bottom_up;
+    const bool quads = may_quad && cnt <= SPREAD_MAX;
     const uint32_t per_pass = gridDim.x * (quads ? DTPB / 4u : (uint32_t)DTPB);
     for (uint32_t it = 0; it * per_pass < cnt; ++it) {
         uint32_t* cur = s_fr;
@@ -1036,7 +1040,7 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
             const uint32_t i = quad_index(it);
             const bool valid = i < cnt;
             const uint32_t u = it == 0 ? first : (valid ? __ldcg(in + i) : 0u);
-            if (__any_sync(0xffffffffu, valid)) bfs_expand_quad(g, valid, u, L, exact, st0, propagate, visits, s_m);
+            if (__any_sync(0xffffffffu, valid)) bfs_expand_quad(g, valid, u, st0, propagate, visits);
         } else {
             const uint32_t i = queue_index(it, cnt);
             if (i < cnt) {
@@ -1053,12 +1057,12 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
             // the slot after next was read before the last block barrier
             if (threadIdx.x == 0) s_m[SUB + (nx == 2u ? 0u : nx + 1u)] = 0u;
             const Stage st{nxt, &s_m[SUB + nx], half, gcnt, out};
-            if (g.inm && c <= QUAD_MAX) {
+            if (may_quad && c <= BFS_QUAD_MAX) {
                 // a warp without a node has nothing to do
                 for (uint32_t j0 = (threadIdx.x >> 5) * 8u; j0 < c; j0 += DTPB / 4u) {
                     const uint32_t j = j0 + ((threadIdx.x & 31u) >> 2);
                     const bool valid = j < c;
-                    bfs_expand_quad(g, valid, valid ? cur[j] : 0u, 0u, false, st, propagate, visits, s_m);
+                    bfs_expand_quad(g, valid, valid ? cur[j] : 0u, st, propagate, visits);
                 }
             } else {
                 for (uint32_t j = threadIdx.x; j < c; j += DTPB) {
@@ -1861,7 +1865,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                     // expansions this step: the frontier, then per block and
                     // pass at most one stage half per sub-level
                     const unsigned long long nn = g.n;
-                    const uint32_t per_pass = gridDim.x * (g.inm && cnt <= SPREAD_MAX ? DTPB / 4u : (uint32_t)DTPB);
+                    const uint32_t per_pass = gridDim.x * (g.inm && !g.bottom_up && cnt <= SPREAD_MAX ? DTPB / 4u : (uint32_t)DTPB);
                     const unsigned long long passes = (cnt + per_pass - 1u) / per_pass;
                     const unsigned long long ex_max =
                         cnt + (unsigned long long)(g.bfs_block_levels - 1) * (DTPB * 4u) * gridDim.x * passes;
