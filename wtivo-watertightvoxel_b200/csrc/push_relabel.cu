@@ -989,6 +989,54 @@ __device__ __forceinline__ void stage_push_warp(const SolveView& g, const Stage&
     if (want2) put(i2, v);
 }
 
+// bfs_expand_one for a whole warp, a node per lane (in-arc masks, top-down
+// only): the label atomics of all slots are in flight together, and the warp
+// appends with one shared atomic.
+__device__ __forceinline__ void bfs_expand_warp(const SolveView& g, bool valid, uint32_t u, const Stage& st,
+                                                bool propagate, unsigned long long& visits)
+{
+    u = valid ? u : 0u;
+    const uint32_t cand = ldcg(g.height + u) + 1u;
+    const int4 nb4 = __ldg(g.nbr + u);
+    const uint32_t m = valid ? (uint32_t)__ldcg(g.inm + u) : 0u;
+    uint32_t v[4] = {(uint32_t)nb4.x, (uint32_t)nb4.y, (uint32_t)nb4.z, (uint32_t)nb4.w};
+    uint32_t hv[4], old[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) hv[k] = ((m >> k) & 1u) ? ldcg(g.height + v[k]) : 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        old[k] = 0u;
+        atom_min_if(hv[k] > cand, old[k], g.height + v[k], cand);
+    }
+    visits += valid ? 1ull : 0ull;
+    unsigned b[4];
+    uint32_t total = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        b[k] = __ballot_sync(0xffffffffu, old[k] > cand && (old[k] == UNVIS || propagate));
+        total += (uint32_t)__popc(b[k]);
+    }
+    if (total == 0u) return;
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    uint32_t base = 0;
+    if (lane == 0u) base = atomicAdd(st.cnt, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if ((b[k] >> lane) & 1u) {
+            const uint32_t idx = base + (uint32_t)__popc(b[k] & below);
+            if (idx < st.cap) {
+                st.buf[idx] = v[k];
+            } else {
+                const uint32_t pos = atomicAdd(st.gcnt, 1u);
+                if (pos < g.n) st.out[pos] = v[k];
+                else raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+            }
+        }
+        base += (uint32_t)__popc(b[k]);
+    }
+}
+
 // bfs_expand_one by four lanes, one per slot (in-arc masks, top-down only): the
 // warp holds eight nodes, `valid` where this lane's node exists.
 __device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, uint32_t u, const Stage& st,
@@ -1043,10 +1091,10 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
             if (__any_sync(0xffffffffu, valid)) bfs_expand_quad(g, valid, u, st0, propagate, visits);
         } else {
             const uint32_t i = queue_index(it, cnt);
-            if (i < cnt) {
-                const uint32_t u = __ldcg(in + i);
-                bfs_expand_one(g, u, exact ? L : ldcg(g.height + u), st0, propagate, visits, s_m);
-            }
+            const bool valid = i < cnt;
+            const uint32_t u = valid ? __ldcg(in + i) : 0u;
+            if (may_quad) bfs_expand_warp(g, valid, u, st0, propagate, visits);
+            else if (valid) bfs_expand_one(g, u, exact ? L : ldcg(g.height + u), st0, propagate, visits, s_m);
         }
         __syncthreads();
         uint32_t last = 0;   // ring slot of the last sub-level's count
@@ -1063,6 +1111,11 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
                     const uint32_t j = j0 + ((threadIdx.x & 31u) >> 2);
                     const bool valid = j < c;
                     bfs_expand_quad(g, valid, valid ? cur[j] : 0u, st, propagate, visits);
+                }
+            } else if (may_quad) {
+                for (uint32_t j0 = threadIdx.x & ~31u; j0 < c; j0 += DTPB) {
+                    const uint32_t j = j0 + (threadIdx.x & 31u);
+                    bfs_expand_warp(g, j < c, j < c ? cur[j] : 0u, st, propagate, visits);
                 }
             } else {
                 for (uint32_t j = threadIdx.x; j < c; j += DTPB) {
