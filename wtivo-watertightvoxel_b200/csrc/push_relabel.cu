@@ -1443,6 +1443,121 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
     return next;
 }
 
+// discharge_node for a whole warp, a node per lane, without chaining or warp
+// aggregation: the lanes stay together, and the warp appends what they own with
+// one shared atomic instead of one a node (long lists).
+__device__ __forceinline__ void discharge_warp(const SolveView& g, bool valid, uint32_t v, const Stage& st,
+                                               Work& w)
+{
+    const uint32_t n = g.n;
+    v = valid ? v : 0u;   // lanes without a node read node 0 and do nothing with it
+    uint32_t h = ldcg(g.height + v);
+    long long ex = ldcg(g.excess + v);
+    const int4 nb4 = __ldg(g.nbr + v);
+    const uint4 r4 = __ldcg(reinterpret_cast<const uint4*>(g.res) + v);
+    const uint32_t rv = __ldg(g.rev + v);
+    bool live = valid && h < n && ex > 0;
+    const int nb[4] = {nb4.x, nb4.y, nb4.z, nb4.w};
+    uint32_t r[4] = {r4.x, r4.y, r4.z, r4.w};
+    uint32_t hn[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        hn[k] = (live && nb[k] >= 0) ? ldcg(g.height + nb[k]) : UNVIS;
+        r[k] = nb[k] >= 0 ? r[k] : 0u;
+    }
+    int32_t t = (live && h == 1u) ? ldcg(g.term + v) : 0;
+    const uint32_t h0 = h;
+    const int32_t t0 = t;
+    const bool mine = live;
+    long long pushed = 0;
+    uint32_t own = 0u;   // bit k: a push took ownership of neighbour k
+    w.visits += live ? 1ull : 0ull;
+    for (int step = 0; __any_sync(0xffffffffu, live); ++step) {
+        if (live && t < 0 && h == 1u) {                // v -> sink (.cu:220-236)
+            const long long cap = -(long long)t;
+            const long long d = ex < cap ? ex : cap;
+            t = (int32_t)((long long)t + d);
+            ex -= d;
+            pushed += d;
+            w.sink += (unsigned long long)d;
+            ++w.pushes;
+        }
+        unsigned long long o[4];
+        uint32_t left[4];   // v's residuals as the pushes found them
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            o[k] = 1ull;
+            left[k] = 0xFFFFFFFFu;
+            const bool adm = live && r[k] != 0u && hn[k] < h && ex > 0;
+            const uint32_t d = adm ? (uint32_t)(ex < (long long)r[k] ? ex : (long long)r[k]) : 0u;
+            r[k] -= d;
+            ex -= d;
+            pushed += d;
+            if (d) {
+                ++w.pushes;
+                const uint32_t rk = (rv >> (2 * k)) & 3u;
+                left[k] = atomicSub(g.res + (size_t)v * 4u + k, d);
+                atomicAdd(g.res + (size_t)nb[k] * 4u + rk, d);
+                o[k] = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb[k]), (unsigned long long)d);
+            }
+        }
+        bool fin = true;
+        if (live && ex > 0) {
+            uint32_t mh = (t < 0) ? 0u : UNVIS;        // relabel (.cu:274-301)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (r[k] != 0u && hn[k] < mh) mh = hn[k];
+            ++w.relabels;
+            h = mh == UNVIS ? UNVIS : mh + 1u;
+            fin = h >= n || step + 1 >= g.local_steps;
+        }
+        live = live && !fin;
+        // others only ever raise v's residuals meanwhile
+        if (left[0] < r[0] || left[1] < r[1] || left[2] < r[2] || left[3] < r[3])
+            raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) own |= (uint32_t)(o[k] == 0ull) << k;
+    }
+    unsigned long long self = (unsigned long long)ex;
+    if (mine) {   // release v's excess: its residuals are lowered (discharge_node)
+        if (h != h0) g.height[v] = h;
+        if (t != t0) {
+            g.term[v] = t;
+            __threadfence();   // the next owner reads it
+        }
+        if (pushed)
+            self = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + v), (unsigned long long)(-pushed));
+    }
+    if (mine && h < n && (long long)self - pushed > 0) own |= 16u;   // keeps ownership
+    unsigned b[5];
+    uint32_t total = 0;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        b[k] = __ballot_sync(0xffffffffu, (own >> k) & 1u);
+        total += (uint32_t)__popc(b[k]);
+    }
+    if (total == 0u) return;
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    uint32_t base = 0;
+    if (lane == 0u) base = atomicAdd(st.cnt, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        if ((own >> k) & 1u) {
+            const uint32_t x = k < 4 ? (uint32_t)nb[k < 4 ? k : 0] : v;
+            const uint32_t idx = base + (uint32_t)__popc(b[k] & below);
+            if (idx < st.cap) {
+                st.buf[idx] = x;
+            } else {
+                const uint32_t pos = atomicAdd(st.gcnt, 1u);
+                if (pos < g.n) st.out[pos] = x;
+                else raise_error(g.ctl, (int)GPUPR_ERR_INVARIANT);
+            }
+        }
+        base += (uint32_t)__popc(b[k]);
+    }
+}
+
 // discharge_node by four lanes, one per slot: the warp holds eight nodes,
 // `valid` where this lane's node exists; every lane of the warp calls it.  On a
 // short list a sub-level is one chain of memory round trips (the node's state,
@@ -1575,7 +1690,8 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
     const int hops = narrow ? g.chain_hops : 1;
     const int levels = narrow ? g.dis_levels : g.dis_levels_wide;
     const uint32_t half = stage_cap / 2u;
-    const bool quads = !kAgg && hops <= 1 && levels > 1 && cnt <= SPREAD_MAX;
+    const bool warps = !kAgg && hops <= 1 && levels > 1;
+    const bool quads = warps && cnt <= SPREAD_MAX;
     const uint32_t per_pass = gridDim.x * (quads ? DTPB / 4u : (uint32_t)DTPB);
     for (uint32_t it = 0; it * per_pass < cnt; ++it) {
         uint32_t* cur = s_buf;
@@ -1587,6 +1703,12 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
             const uint32_t v = valid ? __ldcg(in + i) : 0u;
             if (valid && v >= g.n) raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
             if (__any_sync(0xffffffffu, valid)) discharge_quad(g, valid && v < g.n, v, st0, w);
+        } else if (warps) {
+            const uint32_t i = queue_index(it, cnt);
+            const bool valid = i < cnt;
+            const uint32_t v = valid ? __ldcg(in + i) : 0u;
+            if (valid && v >= g.n) raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
+            discharge_warp(g, valid && v < g.n, v, st0, w);
         } else {
             const uint32_t i = queue_index(it, cnt);
             if (i < cnt) {
@@ -1616,6 +1738,11 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
                     const uint32_t j = j0 + ((threadIdx.x & 31u) >> 2);
                     const bool valid = j < c;
                     discharge_quad(g, valid, valid ? cur[j] : 0u, st, w);
+                }
+            } else if (warps) {
+                for (uint32_t j0 = threadIdx.x & ~31u; j0 < c; j0 += DTPB) {
+                    const uint32_t j = j0 + (threadIdx.x & 31u);
+                    discharge_warp(g, j < c, j < c ? cur[j] : 0u, st, w);
                 }
             } else {
                 for (uint32_t j = threadIdx.x; j < c; j += DTPB) discharge_node<kAgg>(g, cur[j], st, false, w);
