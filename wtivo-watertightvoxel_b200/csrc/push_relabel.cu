@@ -217,7 +217,7 @@ __device__ __forceinline__ void queue_tile(const SolveView& g, uint32_t t, uint3
 // With g.arcm (tiled relabels) the pass writes every node's arc mask instead
 // of an in-arc row and queues the tiles holding a seed for tile step
 // `tile_step`; the seeds are not appended to a frontier.
-template <bool kActive>
+template <bool kActive, bool kLean = false>
 __device__ __forceinline__ void bfs_seed_body(const SolveView& g, uint32_t* s_fr, uint32_t* s_act,
                                               uint32_t* s_m, uint32_t tile_step = 0u)
 {
@@ -241,7 +241,7 @@ __device__ __forceinline__ void bfs_seed_body(const SolveView& g, uint32_t* s_fr
             x[j] = (kActive && in[j] && t[j] < 0) ? ldcg(g.excess + v) : 0ll;
             if (in[j]) g.height[v] = (t[j] < 0) ? 1u : UNVIS;
         }
-        if (g.arcm) {
+        if (!kLean && g.arcm) {
             // a warp's 32 nodes lie in one tile (RELABEL_TILE is a multiple of 32)
 #pragma unroll
             for (int j = 0; j < SWEEP_UNROLL; ++j) {
@@ -253,7 +253,7 @@ __device__ __forceinline__ void bfs_seed_body(const SolveView& g, uint32_t* s_fr
             }
             continue;   // no frontier: the tile steps start from the queued tiles
         }
-        if (g.inm) {
+        if (kLean || g.inm) {
 #pragma unroll
             for (int j = 0; j < SWEEP_UNROLL; ++j) {
                 const uint32_t v = base + j * DTPB + threadIdx.x;
@@ -279,7 +279,7 @@ __device__ __forceinline__ void bfs_seed_body(const SolveView& g, uint32_t* s_fr
             s_m[2] = s_m[0]; s_m[3] = s_m[1]; s_m[0] = 0; s_m[1] = 0;
             s_m[4] = s_m[2] ? atomicAdd(&ctl->bfs_cnt[1], s_m[2]) : 0u;
             s_m[5] = s_m[3] ? atomicAdd(&ctl->act_cnt[0], s_m[3]) : 0u;
-            if (g.bottom_up && s_m[2]) atomicAdd(&ctl->lab_cnt[1], s_m[2]);
+            if (!kLean && g.bottom_up && s_m[2]) atomicAdd(&ctl->lab_cnt[1], s_m[2]);
         }
         __syncthreads();
         flush_stage(s_fr, s_m[2], s_m[4], g.fr[1], g.n, ctl);
@@ -339,6 +339,7 @@ __device__ __forceinline__ uint32_t quad_index(uint32_t it)
 // the same pass collects every reached node (label below UNVIS) into
 // cand[0], staged in s_cand (DTPB * SWEEP_UNROLL entries, counters
 // s_m[7..9]): the candidates of the next relabel's bottom-up steps.
+template <bool kLean>
 __device__ __forceinline__ void active_sweep_body(const SolveView& g, uint32_t* s_act, uint32_t* s_cand,
                                                   uint32_t* s_m)
 {
@@ -359,7 +360,7 @@ __device__ __forceinline__ void active_sweep_body(const SolveView& g, uint32_t* 
         for (int j = 0; j < SWEEP_UNROLL; ++j) {
             const bool act = h[j] < g.n && x[j] > 0;
             if (act) s_act[atomicAdd(&s_m[1], 1u)] = base + j * DTPB + threadIdx.x;
-            if (g.bottom_up && h[j] != UNVIS) s_cand[atomicAdd(&s_m[7], 1u)] = base + j * DTPB + threadIdx.x;
+            if (!kLean && g.bottom_up && h[j] != UNVIS) s_cand[atomicAdd(&s_m[7], 1u)] = base + j * DTPB + threadIdx.x;
             if (g.nseg) {
                 // the graph still has work: one store per group of lanes in the same graph
                 const unsigned grp = __match_any_sync(0xffffffffu, act ? sg[j] : 0xFFFFFFFFu);
@@ -370,12 +371,14 @@ __device__ __forceinline__ void active_sweep_body(const SolveView& g, uint32_t* 
         if (threadIdx.x == 0) {
             s_m[3] = s_m[1]; s_m[1] = 0;
             s_m[5] = s_m[3] ? atomicAdd(&ctl->act_cnt[0], s_m[3]) : 0u;
-            s_m[8] = s_m[7]; s_m[7] = 0;
-            s_m[9] = s_m[8] ? atomicAdd(&ctl->cand_build, s_m[8]) : 0u;
+            if (!kLean) {
+                s_m[8] = s_m[7]; s_m[7] = 0;
+                s_m[9] = s_m[8] ? atomicAdd(&ctl->cand_build, s_m[8]) : 0u;
+            }
         }
         __syncthreads();
         flush_stage(s_act, s_m[3], s_m[5], g.act[0], g.n, ctl);
-        if (g.bottom_up) flush_stage(s_cand, s_m[8], s_m[9], g.cand[0], g.n, ctl);
+        if (!kLean && g.bottom_up) flush_stage(s_cand, s_m[8], s_m[9], g.cand[0], g.n, ctl);
         __syncthreads();
     }
 }
@@ -430,7 +433,7 @@ __device__ __forceinline__ int4 residual_in_arcs(const SolveView& g, uint32_t u,
 // queue when it holds excess.  `first` is the thread's first entry (prefetch_entry).
 __device__ __forceinline__ void bfs_level_body(const SolveView& g, uint32_t L, uint32_t cnt,
                                                uint32_t first, uint32_t* s_fr, uint32_t* s_act,
-                                               uint32_t* s_m, unsigned long long& visits)
+                                               uint32_t* s_m, uint32_t& visits)
 {
     Ctl* ctl = g.ctl;
     const uint32_t* in = (L & 1) ? g.fr[1] : g.fr[0];
@@ -520,11 +523,11 @@ __global__ void __launch_bounds__(DTPB) k_bfs_level(SolveView g, uint32_t L)
         else atomicAdd(&ctl->bfs_levels, 1u);
     }
     if (cnt == 0) return;
-    unsigned long long visits = 0;
+    uint32_t visits = 0;
     if (threadIdx.x == 0) { s_m[0] = 0; s_m[1] = 0; }
     __syncthreads();
     bfs_level_body(g, L, cnt, first, s_fr, s_act, s_m, visits);
-    const unsigned long long vs = warp_block_sum(visits, s_red);
+    const unsigned long long vs = warp_block_sum((unsigned long long)visits, s_red);
     if (threadIdx.x == 0 && vs) atomicAdd(&ctl->bfs_visits, vs);
 }
 
@@ -533,8 +536,11 @@ __global__ void __launch_bounds__(DTPB) k_bfs_level(SolveView g, uint32_t L)
 // block barrier.  All three are 0 between passes.
 constexpr uint32_t SUB = 12u;
 
+// A thread's work counters (a thread of the persistent grid stays far below
+// 2^32 of each; they live in registers through the whole solve).
 struct Work {
-    unsigned long long visits = 0, pushes = 0, relabels = 0, sink = 0;
+    uint32_t visits = 0, pushes = 0, relabels = 0;
+    unsigned long long sink = 0;
 };
 
 // Discharge one active node for up to local_steps push/relabel steps
@@ -587,7 +593,7 @@ __device__ __forceinline__ void stage_push(const SolveView& g, const Stage& st, 
 __device__ __forceinline__ void bfs_step_body(const SolveView& g, uint32_t L, uint32_t cnt,
                                               uint32_t first, uint32_t* s_fr,
                                               uint32_t stage_cap, uint32_t* s_m,
-                                              unsigned long long& visits, int hops, bool propagate,
+                                              uint32_t& visits, int hops, bool propagate,
                                               bool exact)
 {
     Ctl* ctl = g.ctl;
@@ -928,7 +934,7 @@ __device__ __forceinline__ void tile_relabel(const SolveView& g, uint32_t t, uin
 // With direction-optimizing relabels, first labels are counted in s_m[6].
 __device__ __forceinline__ void bfs_expand_one(const SolveView& g, uint32_t u, uint32_t hu,
                                                const Stage& st, bool propagate,
-                                               unsigned long long& visits, uint32_t* s_m)
+                                               uint32_t& visits, uint32_t* s_m)
 {
     uint32_t arcs;
     const int4 nb4 = residual_in_arcs(g, u, &arcs);
@@ -993,7 +999,7 @@ __device__ __forceinline__ void stage_push_warp(const SolveView& g, const Stage&
 // only): the label atomics of all slots are in flight together, and the warp
 // appends with one shared atomic.
 __device__ __forceinline__ void bfs_expand_warp(const SolveView& g, bool valid, uint32_t u, const Stage& st,
-                                                bool propagate, unsigned long long& visits)
+                                                bool propagate, uint32_t& visits)
 {
     u = valid ? u : 0u;
     const uint32_t cand = ldcg(g.height + u) + 1u;
@@ -1008,7 +1014,7 @@ __device__ __forceinline__ void bfs_expand_warp(const SolveView& g, bool valid, 
         old[k] = 0u;
         atom_min_if(hv[k] > cand, old[k], g.height + v[k], cand);
     }
-    visits += valid ? 1ull : 0ull;
+    visits += valid ? 1u : 0u;
     unsigned b[4];
     uint32_t total = 0;
 #pragma unroll
@@ -1040,7 +1046,7 @@ __device__ __forceinline__ void bfs_expand_warp(const SolveView& g, bool valid, 
 // bfs_expand_one by four lanes, one per slot (in-arc masks, top-down only): the
 // warp holds eight nodes, `valid` where this lane's node exists.
 __device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, uint32_t u, const Stage& st,
-                                                bool propagate, unsigned long long& visits)
+                                                bool propagate, uint32_t& visits)
 {
     const uint32_t k = threadIdx.x & 3u;
     u = valid ? u : 0u;   // lanes without a node read node 0 and do nothing with it
@@ -1052,7 +1058,7 @@ __device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, 
     const bool lower = arc && ldcg(g.height + v) > cand;
     uint32_t old = 0u;
     atom_min_if(lower, old, g.height + v, cand);
-    visits += (valid && k == 0u) ? 1ull : 0ull;
+    visits += (valid && k == 0u) ? 1u : 0u;
     stage_push_warp(g, st, lower && old > cand && (old == UNVIS || propagate), v);
 }
 
@@ -1066,10 +1072,11 @@ __device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, 
 // `propagate`): a node labelled here before another block reaches it by a
 // shorter path is lowered and expanded again.  Frontier entries may carry
 // different labels: each expansion reads its node's label.
+template <bool kLean>
 __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_t L, uint32_t cnt,
                                                      uint32_t first, uint32_t* s_fr,
                                                      uint32_t stage_cap, uint32_t* s_m,
-                                                     unsigned long long& visits, int levels,
+                                                     uint32_t& visits, int levels,
                                                      bool propagate, bool exact)
 {
     Ctl* ctl = g.ctl;
@@ -1077,7 +1084,7 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
     uint32_t* out = (L & 1) ? g.fr[0] : g.fr[1];
     uint32_t* gcnt = &ctl->bfs_cnt[(L + 1) % 3];
     const uint32_t half = stage_cap / 2u;
-    const bool may_quad = g.inm && !g.bottom_up;
+    const bool may_quad = kLean || (g.inm && !g.bottom_up);
     const bool quads = may_quad && cnt <= SPREAD_MAX;
     const uint32_t per_pass = gridDim.x * (quads ? DTPB / 4u : (uint32_t)DTPB);
     for (uint32_t it = 0; it * per_pass < cnt; ++it) {
@@ -1132,7 +1139,7 @@ __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_
         if (threadIdx.x == 0) {
             s_m[2] = min(s_m[SUB + last], half);
             s_m[4] = s_m[2] ? atomicAdd(gcnt, s_m[2]) : 0u;
-            if (g.bottom_up && s_m[6]) {
+            if (!kLean && g.bottom_up && s_m[6]) {
                 atomicAdd(&ctl->lab_cnt[(L + 1) % 3], s_m[6]);
                 s_m[6] = 0;
             }
@@ -1207,7 +1214,7 @@ constexpr uint32_t RELABEL_TILES_DEFAULT_MIN = 0xFFFFFFFFu;
 // the level in ctl->tail_L.  s_buf holds 2 * TAIL_CAP entries; s_m[10] is the
 // claim counter.
 __device__ void bfs_tail_body(const SolveView& g, uint32_t L0, uint32_t cnt0, uint32_t* s_buf,
-                              uint32_t* s_m, unsigned long long& visits)
+                              uint32_t* s_m, uint32_t& visits)
 {
     Ctl* ctl = g.ctl;
     uint32_t* sA = s_buf;
@@ -1282,7 +1289,7 @@ __device__ void bfs_tail_body(const SolveView& g, uint32_t L0, uint32_t cnt0, ui
 // stage_cap entries each; s_m[0,2,4] stage the frontier, s_m[7..9] the list.
 __device__ __forceinline__ void bfs_bottom_up_body(const SolveView& g, uint32_t L, uint32_t j,
                                                    uint32_t* s_fr, uint32_t* s_keep, uint32_t stage_cap,
-                                                   uint32_t* s_m, unsigned long long& visits)
+                                                   uint32_t* s_m, uint32_t& visits)
 {
     Ctl* ctl = g.ctl;
     const uint32_t* in = g.cand[j & 1u];
@@ -1471,7 +1478,7 @@ __device__ __forceinline__ void discharge_warp(const SolveView& g, bool valid, u
     const bool mine = live;
     long long pushed = 0;
     uint32_t own = 0u;   // bit k: a push took ownership of neighbour k
-    w.visits += live ? 1ull : 0ull;
+    w.visits += live ? 1u : 0u;
     for (int step = 0; __any_sync(0xffffffffu, live); ++step) {
         if (live && t < 0 && h == 1u) {                // v -> sink (.cu:220-236)
             const long long cap = -(long long)t;
@@ -1677,7 +1684,7 @@ __device__ __forceinline__ void discharge_quad(const SolveView& g, bool valid, u
 // stage_cap / 2 entries, ping-pong; entries that overflow a half go straight to
 // the queue.  With chains the round has one level.  `first` is the thread's
 // first entry (prefetch_entry).
-template <bool kAgg>
+template <bool kAgg, bool kLean>
 __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t round, uint32_t cnt,
                                                uint32_t first, uint32_t* s_buf, uint32_t stage_cap,
                                                uint32_t* s_m, Work& w)
@@ -1687,10 +1694,10 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
     uint32_t* out = (round & 1) ? g.act[0] : g.act[1];
     uint32_t* gcnt = &ctl->act_cnt[(round + 1) % 3];
     const bool narrow = cnt <= g.chain_max_active;
-    const int hops = narrow ? g.chain_hops : 1;
+    const int hops = kLean ? 1 : narrow ? g.chain_hops : 1;
     const int levels = narrow ? g.dis_levels : g.dis_levels_wide;
     const uint32_t half = stage_cap / 2u;
-    const bool warps = !kAgg && hops <= 1 && levels > 1;
+    const bool warps = kLean || (!kAgg && hops <= 1 && levels > 1);
     const bool quads = warps && cnt <= SPREAD_MAX;
     const uint32_t per_pass = gridDim.x * (quads ? DTPB / 4u : (uint32_t)DTPB);
     for (uint32_t it = 0; it * per_pass < cnt; ++it) {
@@ -1764,19 +1771,19 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
     }
 }
 
-__device__ __forceinline__ void reduce_work(Ctl* ctl, const Work& w, unsigned long long bfs_visits,
+__device__ __forceinline__ void reduce_work(Ctl* ctl, const Work& w, uint32_t bfs_visits,
                                             unsigned long long* s_red)
 {
     unsigned long long x;
-    x = warp_block_sum(w.visits, s_red);
+    x = warp_block_sum((unsigned long long)w.visits, s_red);
     if (threadIdx.x == 0 && x) atomicAdd(&ctl->node_visits, x);
-    x = warp_block_sum(w.pushes, s_red);
+    x = warp_block_sum((unsigned long long)w.pushes, s_red);
     if (threadIdx.x == 0 && x) atomicAdd(&ctl->pushes, x);
-    x = warp_block_sum(w.relabels, s_red);
+    x = warp_block_sum((unsigned long long)w.relabels, s_red);
     if (threadIdx.x == 0 && x) atomicAdd(&ctl->relabels, x);
     x = warp_block_sum(w.sink, s_red);
     if (threadIdx.x == 0 && x) atomicAdd(&ctl->sink_flow, x);
-    x = warp_block_sum(bfs_visits, s_red);
+    x = warp_block_sum((unsigned long long)bfs_visits, s_red);
     if (threadIdx.x == 0 && x) atomicAdd(&ctl->bfs_visits, x);
 }
 
@@ -1796,8 +1803,8 @@ __global__ void __launch_bounds__(DTPB) k_discharge(SolveView g, uint32_t round)
     Work w;
     if (threadIdx.x < 16) s_m[threadIdx.x] = 0u;
     __syncthreads();
-    discharge_body<false>(g, round, cnt, first, s_buf, DTPB * 5, s_m, w);
-    reduce_work(ctl, w, 0ull, s_red);
+    discharge_body<false, false>(g, round, cnt, first, s_buf, DTPB * 5, s_m, w);
+    reduce_work(ctl, w, 0u, s_red);
 }
 
 // ---------------------------------------------------------------------------
@@ -1864,13 +1871,17 @@ __device__ __forceinline__ void red_release_add(unsigned long long* p, unsigned 
 // An error anywhere sets BAR_ABORT, which ends every wait at once; a wait
 // also ends, with GPUPR_ERR_TIMEOUT, after wait_ns, and block 0 raises the
 // solve's own time limit here.
-__device__ bool grid_barrier(Ctl* ctl, unsigned long long& target, unsigned long long deadline,
-                             unsigned long long wait_ns, int* s_ok)
+struct BarrierState {
+    unsigned long long target, deadline;   // thread 0's: kept out of registers
+    int ok;
+};
+__device__ bool grid_barrier(Ctl* ctl, BarrierState& st, unsigned long long wait_ns)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
-        target += gridDim.x;
-        if (blockIdx.x == 0 && gtimer() > deadline) raise_error(ctl, (int)GPUPR_ERR_TIMEOUT);
+        const unsigned long long target = st.target + gridDim.x;
+        st.target = target;
+        if (blockIdx.x == 0 && gtimer() > st.deadline) raise_error(ctl, (int)GPUPR_ERR_TIMEOUT);
         red_release_add(&ctl->bar, 1ull);
         int ok = 1;
         unsigned long long t0 = 0;
@@ -1891,28 +1902,34 @@ __device__ bool grid_barrier(Ctl* ctl, unsigned long long& target, unsigned long
                 }
             }
         }
-        *s_ok = ok;
+        st.ok = ok;
     }
     __syncthreads();
-    return *s_ok != 0;
+    return st.ok != 0;
 }
 
 // kAgg: warp-aggregated excess atomics in the discharge (an option).
 // kTiles: tiled relabels (g.arcm set), a separate instantiation so that the
 // frontier-step kernel keeps its registers.
-template <bool kAgg, bool kTiles>
+// kLean: the default settings only (in-arc masks, block sub-levels, no chains, no
+// aggregation, no bottom-up or tail steps): without the code of the options the
+// kernel spills less and its instructions stay in the caches
+// (@LEAN@).
+template <bool kAgg, bool kTiles, bool kLean>
 __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, PersistParams p)
 {
     __shared__ __align__(16) uint32_t s_buf[DTPB * 8];   // 16-byte copies land here (tiles)
     __shared__ uint32_t s_m[16];
     __shared__ unsigned long long s_red[DTPB / 32];
-    __shared__ int s_ok;
+    __shared__ BarrierState s_bar;
     Ctl* ctl = g.ctl;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-    const unsigned long long deadline = gtimer() + p.limit_ns;
-    unsigned long long bar_target = 0;
+    if (threadIdx.x == 0) {
+        s_bar.target = 0ull;
+        s_bar.deadline = gtimer() + p.limit_ns;
+    }
     Work w;
-    unsigned long long bfs_visits = 0;
+    uint32_t bfs_visits = 0;
     // tiled relabels: the last tile step (the same in every block), tiles and
     // nodes this block processed, labels this thread lowered
     uint32_t tstep = 0;
@@ -1960,7 +1977,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
             if (v < g.n) g.excess[v] = t[j] > 0 ? (long long)t[j] : 0ll;   // source arc saturated (.cu:69-83)
         }
     }
-    if (grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok)) {
+    if (grid_barrier(ctl, s_bar, p.wait_ns)) {
         unsigned long long rounds_total = 0;
         uint32_t levels_total = 0, relabels = 0;
         bool ok = true;
@@ -1972,8 +1989,8 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
         while (ok) {
             // ---- global relabel (label-correcting steps, reachability exact) ----
             if (lead) s_rel_t0 = gtimer();
-            bfs_seed_body<false>(g, s_buf, s_buf + DTPB * 4, s_m, kTiles ? tstep + 1u : 0u);
-            if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+            bfs_seed_body<false, kLean>(g, s_buf, s_buf + DTPB * 4, s_m, kTiles ? tstep + 1u : 0u);
+            if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
             const uint32_t S0 = tstep + 1u;   // the seeds' tile step
             while (kTiles) {
                 // ---- tile steps (tiled relabels) ----
@@ -1992,7 +2009,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                     ++tprocs;
                     tloads += min(RELABEL_TILE, g.n - (t << RELABEL_TILE_SHIFT));
                 }
-                if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+                if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
                 ++levels_total;
                 ++tsteps;
             }
@@ -2002,7 +2019,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
             uint32_t labelled = 0, bu_j = 0;
             for (; !kTiles;) {
                 const uint32_t* fin = (L & 1) ? g.fr[1] : g.fr[0];
-                const uint32_t first = g.bfs_block_levels > 1 ? prefetch_quad(fin, g.n) : prefetch_entry(fin, g.n);
+                const uint32_t first = kLean || g.bfs_block_levels > 1 ? prefetch_quad(fin, g.n) : prefetch_entry(fin, g.n);
                 const uint32_t cnt = min(vload(&ctl->bfs_cnt[L % 3]), g.n);
                 if (cnt == 0) break;
                 if (lead) ctl->bfs_cnt[(L + 2) % 3] = 0u;
@@ -2010,18 +2027,18 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                 // every decision below is the same in every block: it depends
                 // on counters completed before the last barrier
                 bool bottom_up = false;
-                if (g.bottom_up) {
+                if (!kLean && g.bottom_up) {
                     labelled += vload(&ctl->lab_cnt[L % 3]);
                     if (lead) ctl->lab_cnt[(L + 2) % 3] = 0u;
                     const uint32_t cc = vload(&ctl->cand_cnt);
                     const uint32_t rem = cc > labelled ? cc - labelled : 0u;
                     bottom_up = cc != 0u && (float)rem <= g.bu_ratio * (float)cnt;
                 }
-                if (!g.bottom_up && g.tail_max && cnt <= g.tail_max) {
+                if (!kLean && !g.bottom_up && g.tail_max && cnt <= g.tail_max) {
                     // a short frontier: block 0 runs the next levels alone
                     if (blockIdx.x == 0) bfs_tail_body(g, L, cnt, s_buf, s_m, bfs_visits);
                     exact = false;
-                    if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+                    if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
                     if (lead) {
                         s_step_ns[0] += gtimer() - t_step;
                         ++s_step_cnt[0];
@@ -2036,12 +2053,12 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                     }
                     continue;
                 }
-                if (bottom_up) {
+                if (!kLean && bottom_up) {
                     bfs_bottom_up_body(g, L, bu_j, s_buf, s_buf + DTPB * 4, DTPB * 4, s_m, bfs_visits);
                     ++bu_j;
                     exact = false;
                     if (lead) ++ctl->bu_steps;
-                } else if (g.bfs_block_levels > 1) {
+                } else if (kLean || g.bfs_block_levels > 1) {
                     // expansions this step: the frontier, then per block and
                     // pass at most one stage half per sub-level
                     const unsigned long long nn = g.n;
@@ -2049,7 +2066,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                     const unsigned long long passes = (cnt + per_pass - 1u) / per_pass;
                     const unsigned long long ex_max =
                         cnt + (unsigned long long)(g.bfs_block_levels - 1) * (DTPB * 4u) * gridDim.x * passes;
-                    bfs_step_levels_body(g, L, cnt, first, s_buf, DTPB * 8, s_m, bfs_visits,
+                    bfs_step_levels_body<kLean>(g, L, cnt, first, s_buf, DTPB * 8, s_m, bfs_visits,
                                          g.bfs_block_levels, 4ull * ex_max <= nn, exact);
                     exact = false;
                 } else {
@@ -2062,7 +2079,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                                   exact);
                     if (hops > 1) exact = false;
                 }
-                if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+                if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
                 if (lead) {
                     const int c = cnt <= 1024u ? 0 : (cnt <= 16384u ? 1 : 2);
                     s_step_ns[c] += gtimer() - t_step;
@@ -2079,8 +2096,8 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
             if (!ok) break;
             ++relabels;
             lap(0);
-            active_sweep_body(g, s_buf, s_buf + DTPB * 4, s_m);
-            if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+            active_sweep_body<kLean>(g, s_buf, s_buf + DTPB * 4, s_m);
+            if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
             if (lead) {
                 const unsigned long long t = gtimer();
                 s_win = (unsigned long long)(RELABEL_TIME_RATIO * (float)(t - s_rel_t0));
@@ -2104,7 +2121,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                 }
                 if (lead) ctl->act_cnt[(r + 2) % 3] = 0u;
                 if (lead) s_dr_t0 = gtimer();   // shared: keeps the discharge's registers free
-                discharge_body<kAgg>(g, r, cnt, first, s_buf, DTPB * 8, s_m, w);
+                discharge_body<kAgg, kLean>(g, r, cnt, first, s_buf, DTPB * 8, s_m, w);
                 if (lead) {
                     if (r == 0u) s_win_cnt = cnt;
                     const unsigned long long t = gtimer();
@@ -2117,7 +2134,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                         }
                     }
                 }
-                if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+                if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
                 if (lead) {
                     const int c = cnt <= 4096u ? 0 : (cnt <= 131072u ? 1 : 2);
                     s_dr_ns[c] += gtimer() - s_dr_t0;
@@ -2150,7 +2167,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                 ctl->bu_cnt[0] = ctl->cand_build;
                 ctl->cand_build = 0u;
             }
-            if (!(ok = grid_barrier(ctl, bar_target, deadline, p.wait_ns, &s_ok))) break;
+            if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
             lap(2);
         }
         if (lead) {
@@ -2313,7 +2330,7 @@ SolveOptions resolve_options(const gpupr_solve_options* o, int local_steps_raw, 
 int persistent_blocks_per_sm()
 {
     int bps = 0;
-    GPUPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_solve_persistent<false, false>, DTPB, 0));
+    GPUPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_solve_persistent<false, false, true>, DTPB, 0));
     return bps;
 }
 
@@ -2335,10 +2352,23 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     using Clock = std::chrono::steady_clock;
     int bps = 0;
     const bool agg = opt.discharge_warp_aggregate > 0;
-    const void* kern = g.arcm ? (agg ? (const void*)k_solve_persistent<true, true>
-                                     : (const void*)k_solve_persistent<false, true>)
-                              : (agg ? (const void*)k_solve_persistent<true, false>
-                                     : (const void*)k_solve_persistent<false, false>);
+    TuneEntry te;
+    const bool tuned = tune_lookup(g.n, &te);
+    // Discharge rounds run in block sub-levels; chains (a thread going on from
+    // node to node) are an option and replace the sub-levels of the rounds
+    // they apply to.  A caller's small round limit counts rounds of one
+    // discharge per queued node, so it turns the sub-levels off (a sub-level
+    // round does the work of many; 16384 is far above the rounds any of the
+    // graphs measured needs, at most 3,200 single ones).
+    const bool plain_rounds = opt.max_rounds < 16384ull;
+    const int chain_hops = opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : plain_rounds ? 4 : 1;
+    const bool lean = !agg && g.inm && !g.bottom_up && opt.bfs_tail_max <= 0 && opt.bfs_block_levels != 1 &&
+                      chain_hops <= 1 && !plain_rounds;
+    const void* kern = g.arcm ? (agg ? (const void*)k_solve_persistent<true, true, false>
+                                     : (const void*)k_solve_persistent<false, true, false>)
+                       : agg  ? (const void*)k_solve_persistent<true, false, false>
+                       : lean ? (const void*)k_solve_persistent<false, false, true>
+                              : (const void*)k_solve_persistent<false, false, false>;
     const size_t dsmem = g.arcm ? TILE_SMEM : 0u;
     if (dsmem) GPUPR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
     GPUPR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, DTPB, dsmem));
@@ -2352,8 +2382,6 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     // below 1.5M free nodes, 3 up to ~5M, 4 above (config 1: 3.3 ms at 2,
     // 1.20 at 3; a 5.6M-node torus 5.07 at 3, 4.87 at 4).
     // An autotuned entry for this size class replaces the rule.
-    TuneEntry te;
-    const bool tuned = tune_lookup(g.n, &te);
     const int want = opt.blocks_per_sm > 0 ? opt.blocks_per_sm
                      : tuned                ? te.blocks_per_sm
                      : g.n < 1500000u       ? 2
@@ -2387,14 +2415,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     GPUPR_CUDA(cudaMemsetAsync(g.ctl, 0, sizeof(Ctl), s));
     GPUPR_CUDA(cudaEventRecord(e0, s));
     SolveView gv = g;
-    // Discharge rounds run in block sub-levels; chains (a thread going on from
-    // node to node) are an option and replace the sub-levels of the rounds
-    // they apply to.  A caller's small round limit counts rounds of one
-    // discharge per queued node, so it turns the sub-levels off (a sub-level
-    // round does the work of many; 16384 is far above the rounds any of the
-    // graphs measured needs, at most 3,200 single ones).
-    const bool plain_rounds = opt.max_rounds < 16384ull;
-    gv.chain_hops = opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : plain_rounds ? 4 : 1;
+    gv.chain_hops = chain_hops;
     gv.dis_levels = plain_rounds ? 1 : gv.chain_hops > 1 ? 1 : DIS_LEVELS;
     gv.dis_levels_wide = plain_rounds ? 1 : DIS_LEVELS_WIDE;
     gv.bfs_hops = opt.bfs_chain_hops > 0 ? std::min(opt.bfs_chain_hops, 64) : BFS_CHAIN_HOPS;
