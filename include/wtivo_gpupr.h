@@ -134,7 +134,7 @@ typedef struct {
                                      (one launch per step); persistent: 2 below
                                      500k free nodes, 1 below 10M, else 0.5, and
                                      earlier once a discharge phase has taken
-                                     1.2 times the relabel before it without
+                                     0.9 times the relabel before it without
                                      halving its active nodes */
     int32_t engine;               /* 0 auto (persistent when the device supports
                                      cooperative launch), 1 one launch per BFS
@@ -146,7 +146,7 @@ typedef struct {
     int32_t chain_max_active;     /* ... only in rounds with at most this many
                                      active nodes (default 131072); without
                                      chaining such rounds run 16 sub-levels,
-                                     wider ones 4.  max_rounds below 16384
+                                     wider ones 8.  max_rounds below 16384
                                      counts rounds of one discharge per queued
                                      node and turns the sub-levels off */
     int32_t bfs_bottom_up;        /* persistent engine: 1 = direction-optimizing

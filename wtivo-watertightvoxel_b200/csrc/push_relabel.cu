@@ -317,10 +317,12 @@ __device__ __forceinline__ uint32_t queue_index(uint32_t it, uint32_t cnt)
 // leaves one or two warps walking the node's four slots one after the other,
 // and a sub-level lasts as long as that instruction chain; four lanes do the
 // slots at once (a 200k-node integer graph: 2.7 -> 1.8 ms, an 8M-tet open box
-// 26.6 -> 18.6 ms with the same schedule).  Above three passes of 64 nodes the
-// threads are better spent on more nodes at a time.
+// 26.6 -> 18.6 ms with the same schedule).  Longer lists are better off with more
+// nodes at a time (discharge with 64 / 96 / 192 / 320: 80M-tet knot 76 / 73 / 73 /
+// 75 ms, 64-graph batch 55.1 / 56.7 / 53.9 / 54.1; BFS with 32 / 64 / 96 / 160: the
+// knot 74 / 68 / 73 / 77 ms, 8M-tet box 15.8 / 14.6 / 15.7 / 15.4).
 constexpr uint32_t QUAD_MAX = 192u;
-constexpr uint32_t BFS_QUAD_MAX = 96u;
+constexpr uint32_t BFS_QUAD_MAX = 64u;
 
 // Queue index of a thread's node in pass `it` when four lanes share a node:
 // eight entries per warp, dealt round-robin over the blocks.
@@ -1175,14 +1177,14 @@ constexpr bool BFS_IN_ARC_MASKS_DEFAULT = true;
 // discharges made or left active, level after level.  A short round is a chain
 // of memory round trips, so many levels share one barrier; in a wide round the
 // nodes of other blocks fall behind and excess that would have merged is moved
-// twice, so few do.  Measured on B200 (mean of three seeds, solve time, 8 / 16 /
+// twice, so fewer do.  Measured on B200 (mean of three seeds, solve time, 8 / 16 /
 // 32 levels in short rounds): a 200k-node integer graph 1.80 / 1.74 / 2.12 ms,
-// an 8M-tet open box 19.9 / 18.6 / 18.9 ms; wide rounds of 1 / 4 / 8 / 12
-// levels: an 80M-tet knot 96 / 78 / 90 / 93 ms, 64 graphs of 50k-4M tets 69 /
-// 63 / 62 / 62 ms.  Rounds of up to 32768, 65536, 131072 or 262144 active nodes
-// counted as short: within 3% of each other on all of them.
+// an 8M-tet open box 19.9 / 18.6 / 18.9 ms; wide rounds of 2 / 4 / 8 levels: an
+// 80M-tet knot 77.8 / 73.1 / 71.7 ms, 64 graphs of 50k-4M tets 55.7 / 53.9 / 52.7
+// ms.  Rounds of up to 32768, 65536, 131072 or 262144 active nodes counted as
+// short: within 3% of each other on all of them.
 constexpr int DIS_LEVELS = 16;
-constexpr int DIS_LEVELS_WIDE = 4;
+constexpr int DIS_LEVELS_WIDE = 8;
 constexpr uint32_t DIS_NARROW_MAX = 131072u;
 
 // When a discharge phase ends (persistent engine, besides the work budget and
@@ -1191,11 +1193,13 @@ constexpr uint32_t DIS_NARROW_MAX = 131072u;
 // buys the phase as much time again.  Time spent on relabels and on discharge
 // stays balanced whatever the graph's size and shape: counting rounds or
 // visits alone left a 200k-node integer graph in 1,024 rounds of a few stuck
-// nodes (16.7 ms, 1.8 ms with this rule), and a 12M-node one needs no relabel
-// in its long tail of shrinking rounds (10.6 ms without the second half of the
-// rule, 6.7 ms with it).  Ratios of 0.8 / 1.2 / 1.5 / 2: 3.2M-tet sphere 3.7 /
-// 4.1 / 4.0 / 4.8 ms, 8M-tet box 22.5 / 19.4 / 19.3 / 19.4 ms.
-constexpr float RELABEL_TIME_RATIO = 1.2f;
+// nodes (16.7 ms; 1.8 ms with this rule alone), and a 12M-node one needs no
+// relabel in its long tail of shrinking rounds (10.6 ms without the second half
+// of the rule, 6.7 ms with it).  Ratios of 0.6 / 0.8 / 0.9 / 1.2 / 1.6 (mean of
+// three seeds): 3.2M-tet sphere 2.9 / 3.1 / 3.3 / 3.9 / 4.7 ms, 8M-tet box 17.8 /
+// 17.0 / 15.9 / 16.5 / 16.8, 80M-tet knot 68.5 / 66.6 / 68.7 / 69.4-73 / 77,
+// 12M-node integer graph 8.2 / 6.8 / 6.6 / 6.5 / 6.1.
+constexpr float RELABEL_TIME_RATIO = 0.9f;
 constexpr float RELABEL_GAIN = 2.0f;
 
 // Free nodes from which the persistent engine relabels by tiles by default.
@@ -1867,7 +1871,7 @@ __device__ __forceinline__ void red_release_add(unsigned long long* p, unsigned 
 // cooperative launch).  ctl->bar counts arrivals since the launch; a block's
 // thread 0 adds its arrival with release semantics and polls with acquire
 // loads until the count reaches this barrier's target (kept per block in
-// `target`): one round trip to L2 to arrive, one to see the last arrival.
+// shared memory): one round trip to L2 to arrive, one to see the last arrival.
 // An error anywhere sets BAR_ABORT, which ends every wait at once; a wait
 // also ends, with GPUPR_ERR_TIMEOUT, after wait_ns, and block 0 raises the
 // solve's own time limit here.
@@ -1914,7 +1918,7 @@ __device__ bool grid_barrier(Ctl* ctl, BarrierState& st, unsigned long long wait
 // kLean: the default settings only (in-arc masks, block sub-levels, no chains, no
 // aggregation, no bottom-up or tail steps): without the code of the options the
 // kernel spills less and its instructions stay in the caches
-// (@LEAN@).
+// (spills 128 -> 16 bytes; 64-graph batch 55.4 -> 53.9 ms, 900k-tet box 5.1 -> 4.8 ms).
 template <bool kAgg, bool kTiles, bool kLean>
 __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, PersistParams p)
 {
