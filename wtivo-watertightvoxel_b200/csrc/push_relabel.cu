@@ -1189,8 +1189,10 @@ constexpr uint32_t DIS_NARROW_MAX = 131072u;
 
 // When a discharge phase ends (persistent engine, besides the work budget and
 // the round cap): after RELABEL_TIME_RATIO times what the relabel before it
-// took, unless the active nodes fell to 1/RELABEL_GAIN in that time, which
-// buys the phase as much time again.  Time spent on relabels and on discharge
+// took and RELABEL_MIN_ROUNDS rounds, unless the active nodes fell to
+// 1/RELABEL_GAIN in that time, which buys the phase as much again (a relabel of a
+// 330k-node integer graph takes about one round: 1.49 ms without the least number
+// of rounds, 1.15 ms with it).  Time spent on relabels and on discharge
 // stays balanced whatever the graph's size and shape: counting rounds or
 // visits alone left a 200k-node integer graph in 1,024 rounds of a few stuck
 // nodes (16.7 ms; 1.8 ms with this rule alone), and a 12M-node one needs no
@@ -1201,6 +1203,7 @@ constexpr uint32_t DIS_NARROW_MAX = 131072u;
 // 12M-node integer graph 8.2 / 6.8 / 6.6 / 6.5 / 6.1.
 constexpr float RELABEL_TIME_RATIO = 0.9f;
 constexpr float RELABEL_GAIN = 2.0f;
+constexpr uint32_t RELABEL_MIN_ROUNDS = 3u;
 
 // Free nodes from which the persistent engine relabels by tiles by default.
 constexpr uint32_t RELABEL_TILES_DEFAULT_MIN = 0xFFFFFFFFu;
@@ -1959,7 +1962,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
     __shared__ unsigned long long s_dr_ns[3], s_dr_t0;
     __shared__ uint32_t s_dr_cnt[3];
     __shared__ unsigned long long s_rel_t0, s_dr_limit, s_win;
-    __shared__ uint32_t s_win_cnt;
+    __shared__ uint32_t s_win_cnt, s_win_r;
     auto lap = [&](int phase) {
         if (lead) {
             const unsigned long long t = gtimer();
@@ -2127,11 +2130,15 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                 if (lead) s_dr_t0 = gtimer();   // shared: keeps the discharge's registers free
                 discharge_body<kAgg, kLean>(g, r, cnt, first, s_buf, DTPB * 8, s_m, w);
                 if (lead) {
-                    if (r == 0u) s_win_cnt = cnt;
+                    if (r == 0u) {
+                        s_win_cnt = cnt;
+                        s_win_r = 0u;
+                    }
                     const unsigned long long t = gtimer();
-                    if (t > s_dr_limit) {
+                    if (t > s_dr_limit && r + 1u >= s_win_r + RELABEL_MIN_ROUNDS) {
                         if ((float)cnt * RELABEL_GAIN <= (float)s_win_cnt) {
                             s_win_cnt = cnt;
+                            s_win_r = r + 1u;
                             s_dr_limit = t + s_win;
                         } else {
                             ctl->stop_round = (uint32_t)rounds_total + 1u;
