@@ -147,8 +147,9 @@ typedef struct {
                                      active nodes (default 131072); without
                                      chaining such rounds run 16 sub-levels,
                                      wider ones 8.  max_rounds below 16384
-                                     counts rounds of one discharge per queued
-                                     node and turns the sub-levels off */
+                                     and a global_relabel_period of 1 to 63
+                                     count rounds of one discharge per queued
+                                     node and turn the sub-levels off */
     int32_t bfs_bottom_up;        /* persistent engine: 1 = direction-optimizing
                                      global relabels (bottom-up steps over the
                                      nodes the previous relabel reached and this

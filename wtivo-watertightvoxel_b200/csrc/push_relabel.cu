@@ -2367,11 +2367,12 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     const bool tuned = tune_lookup(g.n, &te);
     // Discharge rounds run in block sub-levels; chains (a thread going on from
     // node to node) are an option and replace the sub-levels of the rounds
-    // they apply to.  A caller's small round limit counts rounds of one
-    // discharge per queued node, so it turns the sub-levels off (a sub-level
-    // round does the work of many; 16384 is far above the rounds any of the
-    // graphs measured needs, at most 3,200 single ones).
-    const bool plain_rounds = opt.max_rounds < 16384ull;
+    // they apply to.  A caller's small round limit or relabel period counts
+    // rounds of one discharge per queued node, so it turns the sub-levels off
+    // (a sub-level round does the work of up to 16; 16384 rounds are far above
+    // what any of the graphs measured needs, at most 3,200 single ones, and 64
+    // sub-level rounds are as much as the default period of 1024 single ones).
+    const bool plain_rounds = opt.max_rounds < 16384ull || (opt.period > 0 && opt.period < 64);
     const int chain_hops = opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : plain_rounds ? 4 : 1;
     const bool lean = !agg && g.inm && !g.bottom_up && opt.bfs_tail_max <= 0 && opt.bfs_block_levels != 1 &&
                       chain_hops <= 1 && !plain_rounds;
