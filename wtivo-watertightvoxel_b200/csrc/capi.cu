@@ -401,23 +401,16 @@ void prepare_batch(uint32_t G, const uint64_t* toff, const uint64_t* voff, const
     build_reduced_graph(in, pb.g, pb.info, s, launches);
     if (pb.info.free_n == 0) return;
     // each graph's free nodes form one contiguous range of reduced ids
-    DevBuf<unsigned long long> counts(G, s);
-    batch_free_counts(G, pb.d_toff.p, pb.g.full_to_free.p, counts.p, s, launches);
-    pb.hc.assign(G, 0);
-    std::vector<unsigned long long> hfo(G + 1);
-    std::vector<uint32_t> hso(G + 1);
-    GPUPR_CUDA(cudaMemcpyAsync(pb.hc.data(), counts.p, G * 8u, cudaMemcpyDeviceToHost, s));
-    GPUPR_CUDA(cudaStreamSynchronize(s));
-    hfo[0] = 0;
-    for (uint32_t k = 0; k < G; ++k) hfo[k + 1] = hfo[k] + pb.hc[k];
-    if (hfo[G] != pb.g.n) throw Error{GPUPR_ERR_INVARIANT, "batch free counts do not add up"};
-    for (uint32_t k = 0; k <= G; ++k) hso[k] = (uint32_t)hfo[k];
     pb.d_foff = DevBuf<unsigned long long>(G + 1, s);
     pb.d_soff = DevBuf<uint32_t>(G + 1, s);
-    GPUPR_CUDA(cudaMemcpyAsync(pb.d_foff.p, hfo.data(), (G + 1) * 8u, cudaMemcpyHostToDevice, s));
-    GPUPR_CUDA(cudaMemcpyAsync(pb.d_soff.p, hso.data(), (G + 1) * 4u, cudaMemcpyHostToDevice, s));
-    // the host vectors go out of scope: the copies must have read them
+    batch_free_offsets(G, pb.g.n, pb.d_toff.p, pb.g.free_old.p, pb.d_foff.p, pb.d_soff.p, s, launches);
+    std::vector<unsigned long long> hfo(G + 1);
+    GPUPR_CUDA(cudaMemcpyAsync(hfo.data(), pb.d_foff.p, (G + 1) * 8u, cudaMemcpyDeviceToHost, s));
     GPUPR_CUDA(cudaStreamSynchronize(s));
+    if (hfo[0] != 0 || hfo[G] != pb.g.n)
+        throw Error{GPUPR_ERR_INVARIANT, "batch free counts do not add up"};
+    pb.hc.resize(G);
+    for (uint32_t k = 0; k < G; ++k) pb.hc[k] = hfo[k + 1] - hfo[k];
     pb.segs.nseg = G;
     pb.segs.d_off = pb.d_soff.p;
 }
@@ -509,7 +502,7 @@ void run_graph_cut_batch(uint32_t G, const uint64_t* toff, const uint64_t* voff,
     DevBuf<long long> raw(G, s);
     std::vector<unsigned long long> hb(G);
     std::vector<long long> hr(G);
-    batch_flows(G, pb.d_foff.p, g.term.p, w.excess.p, g.base_node.p, raw.p, base.p, s, &launches);
+    batch_flows(G, g.n, pb.d_foff.p, g.term.p, w.excess.p, g.base_node.p, raw.p, base.p, s, &launches);
     GPUPR_CUDA(cudaMemcpyAsync(hr.data(), raw.p, G * 8u, cudaMemcpyDeviceToHost, s));
     GPUPR_CUDA(cudaMemcpyAsync(hb.data(), base.p, G * 8u, cudaMemcpyDeviceToHost, s));
     if (!out_dev) device_to_host(out, d_out, N, s);

@@ -270,9 +270,10 @@ void batch_pack(uint64_t N, uint32_t G, const unsigned long long* d_tet_off,
                 const unsigned long long* d_vert_off, const int32_t* d_tets_local,
                 const int32_t* d_nbrs_local, int32_t* d_tets, int32_t* d_nbrs, cudaStream_t s,
                 uint64_t* launches);
-void batch_free_counts(uint32_t G, const unsigned long long* d_tet_off, const int32_t* d_full_to_free,
-                       unsigned long long* d_counts, cudaStream_t s, uint64_t* launches);
-void batch_flows(uint32_t G, const unsigned long long* d_free_off, const int32_t* d_term,
+void batch_free_offsets(uint32_t G, uint32_t F, const unsigned long long* d_tet_off,
+                        const uint32_t* d_free_old, unsigned long long* d_free_off,
+                        uint32_t* d_seg_off, cudaStream_t s, uint64_t* launches);
+void batch_flows(uint32_t G, uint32_t n, const unsigned long long* d_free_off, const int32_t* d_term,
                  const long long* d_excess, const uint32_t* d_base_node, long long* d_raw,
                  unsigned long long* d_base, cudaStream_t s, uint64_t* launches);
 
