@@ -10,8 +10,8 @@
 //   k_tile_scan  exclusive scan of the tile counts  (serial compaction :179-187)
 //   k_assign     reduced id = rank among free tets in tet order
 //   k_build_rows per free tet: 4 capacities (bit-exact FP64, :65-98), ELL row,
-//                reverse-slot codes, arc-pair capacity sums, t-link sums,
-//                base flow (:253-291)
+//                t-link sums, base flow (:253-291)
+//   k_reverse_slots  per free tet: reverse-slot codes, arc-pair capacity sums
 //
 // Layout written to HBM (SoA, one 16-byte row per free node):
 //   nbr int4[F], res uint4[F], rev uint8[F] (2 bits per slot),
@@ -185,44 +185,24 @@ __device__ __forceinline__ bool face_capacity(const double (&P)[4][3], uint8_t l
     return true;
 }
 
-// Capacity of face rk of tet j in j's own direction, computed exactly as the
-// thread that builds j's row computes it (same vertex order, same rounding):
-// the face's three vertices go to positions 0,1,2 in the order face slot rk
-// takes them, and face_capacity<0> runs the same operations on them.
-__device__ __forceinline__ uint32_t reverse_capacity(const double* __restrict__ V, uint64_t nv,
-                                                     int4 tj4, int rk, uint8_t lj, uint8_t li,
-                                                     double fill_T)
-{
-    const int tj[4] = {tj4.x, tj4.y, tj4.z, tj4.w};
-    const int ia = (rk == 3) ? 1 : 0;
-    const int ib = (rk <= 1) ? 1 : 2;
-    const int ic = (rk == 0) ? 2 : 3;
-    const int pick[3] = {tj[ia], tj[ib], tj[ic]};
-    double Q[4][3];
-    Q[3][0] = Q[3][1] = Q[3][2] = 0.0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        if (pick[k] < 0 || (uint64_t)pick[k] >= nv) return 0u;   // j's own row reports it
-        const double* p = V + (size_t)pick[k] * 3u;
-        Q[k][0] = __ldg(p);
-        Q[k][1] = __ldg(p + 1);
-        Q[k][2] = __ldg(p + 2);
-    }
-    int32_t cap = 0;
-    if (!face_capacity<0>(Q, lj, li, fill_T, &cap)) return 0u;
-    return (uint32_t)cap;
-}
-
-__global__ void __launch_bounds__(TPB) k_build_rows(
+// Bound by the gathers (per slot the neighbour's label and id, per tet four
+// vertices) and the FP64 capacities, four a tet.  The pair sums need the
+// neighbour's capacity in its own direction, whose vertex order rounds
+// differently: k_reverse_slots reads it from the finished rows.  Computing it
+// a second time here took twice the FP64 work and the neighbours' tet and
+// adjacency rows (24M-tet torus knot: 1235 us for all, now 490 and 290 for the
+// pass over the rows).  Four blocks an SM at 64 registers with 32 bytes of
+// spills: 490 us, three at 78 without: 595.
+__global__ void __launch_bounds__(TPB, 4) k_build_rows(
     uint32_t F, uint64_t N, const double* __restrict__ V, uint64_t nv,
     const int4* __restrict__ tets, const int4* __restrict__ nbrs,
     const uint8_t* __restrict__ labels, const int32_t* __restrict__ full_to_free,
     const uint32_t* __restrict__ free_old, double fill_T, int4* __restrict__ out_nbr,
-    uint4* __restrict__ out_res, uint8_t* __restrict__ out_rev, uint4* __restrict__ out_pair,
-    int32_t* __restrict__ out_term, uint32_t* __restrict__ out_base, BuildCtl* ctl)
+    uint4* __restrict__ out_res, int32_t* __restrict__ out_term, uint32_t* __restrict__ out_base,
+    BuildCtl* ctl)
 {
     __shared__ unsigned long long sh[TPB / 32];
-    unsigned long long refs = 0, terms = 0;
+    uint32_t refs = 0, terms = 0;   // at most 4 a node, a few thousand nodes a thread
     long long base = 0;
     for (uint32_t q = blockIdx.x * TPB + threadIdx.x; q < F; q += gridDim.x * TPB) {
         const uint32_t i = __ldg(free_old + q);
@@ -241,71 +221,50 @@ __global__ void __launch_bounds__(TPB) k_build_rows(
             P[k][1] = __ldg(p + 1);
             P[k][2] = __ldg(p + 2);
         }
-        long long src = 0, snk = 0;
-        int on[4] = {-1, -1, -1, -1};
-        uint32_t orr[4] = {0u, 0u, 0u, 0u};
-        uint32_t opr[4] = {0u, 0u, 0u, 0u};
-        uint32_t rv = 0;
-        int32_t caps[4];
+        uint32_t src = 0, snk = 0;   // four capacities below 2^30 each
+        int on[4];
+        uint32_t orr[4];
         int32_t ms[4];
         uint8_t lj[4];
 #pragma unroll
-        for (int fi = 0; fi < 4; ++fi) lj[fi] = __ldg(labels + row[fi]);
-        ok &= face_capacity<0>(P, li, lj[0], fill_T, &caps[0]);
-        ok &= face_capacity<1>(P, li, lj[1], fill_T, &caps[1]);
-        ok &= face_capacity<2>(P, li, lj[2], fill_T, &caps[2]);
-        ok &= face_capacity<3>(P, li, lj[3], fill_T, &caps[3]);
-#pragma unroll
-        for (int fi = 0; fi < 4; ++fi) ms[fi] = __ldg(full_to_free + row[fi]);
-#pragma unroll
-        for (int fi = 0; fi < 4; ++fi) {
-            const int j = row[fi];  // free tets have no -1 slot and j < N
-            const int32_t m = ms[fi];
-            const int32_t cap = caps[fi];
-            if (m >= 0) {
-                on[fi] = m;
-                orr[fi] = (uint32_t)cap;
-                ++refs;
-                const int4 back = __ldg(nbrs + j);
-                int rk = -1;
-                if (back.w == (int)i) rk = 3;
-                if (back.z == (int)i) rk = 2;
-                if (back.y == (int)i) rk = 1;
-                if (back.x == (int)i) rk = 0;
-                if (rk < 0) {
-                    atomicExch(&ctl->err_reverse, 1);
-                    atomicExch(&ctl->err_node, i);
-                    rk = 0;
-                }
-                rv |= (uint32_t)rk << (2 * fi);
-                // both caps are below 2^30, so the sum fits 32 bits
-                opr[fi] = (uint32_t)cap + reverse_capacity(V, nv, __ldg(tets + j), rk, lj[fi], li,
-                                                           fill_T);
-            } else if (m == -2) {
-                src += cap;
-                ++terms;
-            } else {
-                snk += cap;
-                ++terms;
-            }
+        for (int fi = 0; fi < 4; ++fi) {   // free tets have no -1 slot, all are < N
+            lj[fi] = __ldg(labels + row[fi]);
+            ms[fi] = __ldg(full_to_free + row[fi]);
         }
-        const long long diff = src - snk;
+        auto slot = [&](int fi, bool valid, int32_t cap) {
+            ok &= valid;
+            const int32_t m = ms[fi];
+            on[fi] = m >= 0 ? m : -1;
+            orr[fi] = m >= 0 ? (uint32_t)cap : 0u;
+            refs += m >= 0;
+            terms += m < 0;
+            if (m == -2) src += (uint32_t)cap;
+            else if (m < 0) snk += (uint32_t)cap;
+        };
+        int32_t cap = 0;
+        bool valid = face_capacity<0>(P, li, lj[0], fill_T, &cap);
+        slot(0, valid, cap);
+        valid = face_capacity<1>(P, li, lj[1], fill_T, &cap);
+        slot(1, valid, cap);
+        valid = face_capacity<2>(P, li, lj[2], fill_T, &cap);
+        slot(2, valid, cap);
+        valid = face_capacity<3>(P, li, lj[3], fill_T, &cap);
+        slot(3, valid, cap);
+        const long long diff = (long long)src - (long long)snk;
         if (diff < -2147483648LL || diff > 2147483647LL) ok = false;
         if (!ok) {
             atomicExch(&ctl->err_build, 1);
             atomicExch(&ctl->err_node, i);
         }
         base += (src < snk) ? src : snk;
-        if (out_base) out_base[q] = (uint32_t)((src < snk) ? src : snk);
+        if (out_base) out_base[q] = (src < snk) ? src : snk;
         out_nbr[q] = make_int4(on[0], on[1], on[2], on[3]);
         out_res[q] = make_uint4(orr[0], orr[1], orr[2], orr[3]);
-        out_rev[q] = (uint8_t)rv;
-        out_pair[q] = make_uint4(opr[0], opr[1], opr[2], opr[3]);
         out_term[q] = (int32_t)diff;
     }
-    const unsigned long long r = block_sum(refs, sh);
+    const unsigned long long r = block_sum((unsigned long long)refs, sh);
     if (threadIdx.x == 0 && r) atomicAdd(&ctl->free_refs, r);
-    const unsigned long long t = block_sum(terms, sh);
+    const unsigned long long t = block_sum((unsigned long long)terms, sh);
     if (threadIdx.x == 0 && t) atomicAdd(&ctl->terminal_edges, t);
     const long long b = block_sum(base, reinterpret_cast<long long*>(sh));
     if (threadIdx.x == 0 && b) atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->base_flow), (unsigned long long)b);
@@ -313,35 +272,50 @@ __global__ void __launch_bounds__(TPB) k_build_rows(
 
 // Reverse slots and arc-pair residual sums of a graph in the reference
 // layout.  A pair sum above 2^32 - 1 (residuals the solver's uint32 arcs
-// cannot hold once pushed) is reported as GPUPR_ERR_BUILD.
+// cannot hold once pushed) is reported as GPUPR_ERR_BUILD.  Bound by the
+// gathered rows: both rows of all four neighbours are asked for before the
+// first is looked at, so a node waits for memory twice, not once a slot and
+// again for the residual the slot selects (which sits in the sector a 16-byte
+// row load brings in anyway).  node_id, where given, names the node in
+// *err_node.
 __global__ void __launch_bounds__(TPB) k_reverse_slots(uint32_t n, const int4* __restrict__ nbr,
                                                        const uint4* __restrict__ res,
                                                        uint8_t* __restrict__ rev,
-                                                       uint4* __restrict__ pair, int32_t* err)
+                                                       uint4* __restrict__ pair, int32_t* err,
+                                                       const uint32_t* __restrict__ node_id,
+                                                       uint32_t* err_node)
 {
     for (uint32_t v = blockIdx.x * TPB + threadIdx.x; v < n; v += gridDim.x * TPB) {
         const int4 r4 = __ldg(nbr + v);
         const uint4 c4 = __ldg(res + v);
         const int row[4] = {r4.x, r4.y, r4.z, r4.w};
         const uint32_t own[4] = {c4.x, c4.y, c4.z, c4.w};
+        int4 b[4];
+        uint4 c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool in = (uint32_t)row[k] < n;   // a negative id is above n as well
+            b[k] = in ? __ldg(nbr + row[k]) : make_int4(-1, -1, -1, -1);
+            c[k] = in ? __ldg(res + row[k]) : make_uint4(0u, 0u, 0u, 0u);
+        }
         uint32_t rv = 0;
         uint32_t pr[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int u = row[k];
-            if (u < 0) continue;
-            if ((uint32_t)u >= n) { atomicExch(err, (int)GPUPR_ERR_INVARIANT); continue; }
-            const int4 b = __ldg(nbr + u);
-            int rk = -1;
-            if (b.w == (int)v) rk = 3;
-            if (b.z == (int)v) rk = 2;
-            if (b.y == (int)v) rk = 1;
-            if (b.x == (int)v) rk = 0;
-            if (rk < 0) { atomicExch(err, (int)GPUPR_ERR_NO_REVERSE); rk = 0; }
-            rv |= (uint32_t)rk << (2 * k);
-            const unsigned long long sum =
-                (unsigned long long)own[k] +
-                __ldg(reinterpret_cast<const uint32_t*>(res) + (size_t)u * 4u + rk);
+            if (row[k] < 0) continue;
+            if ((uint32_t)row[k] >= n) { atomicExch(err, (int)GPUPR_ERR_INVARIANT); continue; }
+            uint32_t rk = 0u, back = c[k].x;
+            if (b[k].x != (int)v) {
+                if (b[k].y == (int)v) { rk = 1u; back = c[k].y; }
+                else if (b[k].z == (int)v) { rk = 2u; back = c[k].z; }
+                else if (b[k].w == (int)v) { rk = 3u; back = c[k].w; }
+                else {
+                    atomicExch(err, (int)GPUPR_ERR_NO_REVERSE);
+                    if (node_id) atomicExch(err_node, __ldg(node_id + v));
+                }
+            }
+            rv |= rk << (2 * k);
+            const unsigned long long sum = (unsigned long long)own[k] + back;
             if (sum > 0xFFFFFFFFull) { atomicExch(err, (int)GPUPR_ERR_BUILD); continue; }
             pr[k] = (uint32_t)sum;
         }
@@ -450,10 +424,13 @@ void build_reduced_graph(const BuildInputs& in, ReducedGraph& g, BuildInfo& info
     k_build_rows<<<grid_for(F), TPB, 0, s>>>(
         F, N, in.d_vertices, in.nv, reinterpret_cast<const int4*>(in.d_tets),
         reinterpret_cast<const int4*>(in.d_nbrs), in.d_labels, g.full_to_free.p, g.free_old.p,
-        in.fill_T, g.nbr.p, reinterpret_cast<uint4*>(g.res.p), g.rev.p,
-        reinterpret_cast<uint4*>(g.pair.p), g.term.p, g.base_node.p, ctl.p);
+        in.fill_T, g.nbr.p, reinterpret_cast<uint4*>(g.res.p), g.term.p, g.base_node.p, ctl.p);
     GPUPR_CUDA(cudaGetLastError());
-    *launches += 1;
+    k_reverse_slots<<<grid_for(F), TPB, 0, s>>>(F, g.nbr.p, reinterpret_cast<const uint4*>(g.res.p),
+                                                g.rev.p, reinterpret_cast<uint4*>(g.pair.p),
+                                                &ctl.p->err_reverse, g.free_old.p, &ctl.p->err_node);
+    GPUPR_CUDA(cudaGetLastError());
+    *launches += 2;
     GPUPR_CUDA(cudaMemcpyAsync(&h, ctl.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     GPUPR_CUDA(cudaStreamSynchronize(s));
     if (h.err_build) throw Error{GPUPR_ERR_BUILD, "invalid graph reduction/capacity state"};
@@ -493,7 +470,8 @@ void compute_reverse_slots(uint32_t n, const int4* d_nbr, const uint32_t* d_res,
     DevBuf<int32_t> err(1, s);
     GPUPR_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int32_t), s));
     k_reverse_slots<<<grid_for(n), TPB, 0, s>>>(n, d_nbr, reinterpret_cast<const uint4*>(d_res),
-                                                d_rev, reinterpret_cast<uint4*>(d_pair), err.p);
+                                                d_rev, reinterpret_cast<uint4*>(d_pair), err.p, nullptr,
+                                                nullptr);
     GPUPR_CUDA(cudaGetLastError());
     *launches += 1;
     int32_t e = 0;
@@ -532,7 +510,8 @@ void compute_reverse_slots_noalloc(uint32_t n, const int4* d_nbr, const uint32_t
 {
     GPUPR_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int32_t), s));
     k_reverse_slots<<<grid_for(n), TPB, 0, s>>>(n, d_nbr, reinterpret_cast<const uint4*>(d_res),
-                                                d_rev, reinterpret_cast<uint4*>(d_pair), d_err);
+                                                d_rev, reinterpret_cast<uint4*>(d_pair), d_err, nullptr,
+                                                nullptr);
     GPUPR_CUDA(cudaGetLastError());
     int32_t e = 0;
     GPUPR_CUDA(cudaMemcpyAsync(&e, d_err, sizeof(e), cudaMemcpyDeviceToHost, s));
