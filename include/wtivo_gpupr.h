@@ -139,17 +139,16 @@ typedef struct {
     int32_t engine;               /* 0 auto (persistent when the device supports
                                      cooperative launch), 1 one launch per BFS
                                      level / round, 2 persistent */
-    int32_t chain_hops;           /* persistent engine: nodes one thread may
-                                     discharge in a row in one round, instead of
-                                     the round's block sub-levels (default 1 = no
-                                     chaining) */
-    int32_t chain_max_active;     /* ... only in rounds with at most this many
-                                     active nodes (default 131072); without
-                                     chaining such rounds run 16 sub-levels,
-                                     wider ones 8.  max_rounds below 16384
-                                     and a global_relabel_period of 1 to 63
-                                     count rounds of one discharge per queued
-                                     node and turn the sub-levels off */
+    int32_t chain_hops;           /* persistent engine: nodes excess may travel in
+                                     one short round, where above the round's 16
+                                     block sub-levels */
+    int32_t chain_max_active;     /* persistent engine: rounds with at most this
+                                     many active nodes are short (default
+                                     131072); wider ones run 8 sub-levels.
+                                     max_rounds below 16384 and a
+                                     global_relabel_period of 1 to 63 count
+                                     smaller rounds: chain_hops sub-levels
+                                     (default 4) short, one wide */
     int32_t bfs_bottom_up;        /* persistent engine: 1 = direction-optimizing
                                      global relabels (bottom-up steps over the
                                      nodes the previous relabel reached and this

@@ -112,12 +112,9 @@ struct SolveView {
     uint32_t* fr[2];                    // BFS frontiers (fr[1] aliases act[1])
     Ctl* ctl;
     int local_steps;
-    int chain_hops;                     // nodes one thread may discharge in a row in
-                                        // one round (<= 1: no chaining) ...
-    uint32_t chain_max_active;          // ... in rounds of at most this many nodes (the
-                                        // short rounds)
-    int dis_levels;                     // persistent engine: levels of a discharge round of at
-                                        // most chain_max_active nodes (1: no sub-levels) ...
+    uint32_t chain_max_active;          // discharge rounds of at most this many nodes are short
+    int dis_levels;                     // persistent engine: levels of a short discharge round
+                                        // (1: no sub-levels) ...
     int dis_levels_wide;                // ... and of a wider one
     int bfs_block_levels;               // persistent engine: > 1 = BFS steps expand that many
                                         // levels per block from its shared stage (0: chains)

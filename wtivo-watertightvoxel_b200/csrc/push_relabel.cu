@@ -1200,10 +1200,16 @@ constexpr uint32_t DIS_NARROW_MAX = 131072u;
 // of the rule, 6.7 ms with it).  Ratios of 0.6 / 0.8 / 0.9 / 1.2 / 1.6 (mean of
 // three seeds): 3.2M-tet sphere 2.9 / 3.1 / 3.3 / 3.9 / 4.7 ms, 8M-tet box 17.8 /
 // 17.0 / 15.9 / 16.5 / 16.8, 80M-tet knot 68.5 / 66.6 / 68.7 / 69.4-73 / 77,
-// 12M-node integer graph 8.2 / 6.8 / 6.6 / 6.5 / 6.1.
+// 12M-node integer graph 8.2 / 6.8 / 6.6 / 6.5 / 6.1.  Gains of 2 / 1.5 / 1.25:
+// a 2.4M-node integer graph 4.4 / 3.0 / 3.1 ms, a 5M-node one 5.1 / 4.6 / 4.5, the
+// 3.2M-tet sphere 2.7 / 2.9 / 3.2, a 2.6M-tet box 15.4 / 15.6 / 17.9, equal within
+// the spread of a variant's own runs over 32 graphs.  Where the caller's limits count
+// smaller rounds (plain_rounds below), the least number is RELABEL_MIN_ROUNDS_SINGLE: a
+// graph that needs no second relabel is done by then.
 constexpr float RELABEL_TIME_RATIO = 0.9f;
-constexpr float RELABEL_GAIN = 2.0f;
+constexpr float RELABEL_GAIN = 1.5f;
 constexpr uint32_t RELABEL_MIN_ROUNDS = 3u;
+constexpr uint32_t RELABEL_MIN_ROUNDS_SINGLE = 256u;
 
 // Free nodes from which the persistent engine relabels by tiles by default.
 constexpr uint32_t RELABEL_TILES_DEFAULT_MIN = 0xFFFFFFFFu;
@@ -1345,13 +1351,9 @@ __device__ __forceinline__ void bfs_bottom_up_body(const SolveView& g, uint32_t 
     }
 }
 
-// Returns the node to discharge next in the same round (chaining: a node
-// whose excess this discharge moved from 0 up is owned by this thread, and
-// instead of queueing it for the next round the thread may carry on with
-// it, so excess can travel several hops per round), or UNVIS.
-template <bool kAgg>
-__device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t v, const Stage& st,
-                                                   bool may_chain, Work& w)
+// Discharges one node per thread, with warp aggregation (the option's long
+// lists; without it discharge_warp takes them).
+__device__ __forceinline__ void discharge_node(const SolveView& g, uint32_t v, const Stage& st, Work& w)
 {
     const uint32_t n = g.n;
     // every load of the node's own state is issued before any test, so they
@@ -1362,11 +1364,10 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
     const int4 nb4 = __ldg(g.nbr + v);
     const uint4 r4 = __ldcg(reinterpret_cast<const uint4*>(g.res) + v);
     const uint32_t rv = __ldg(g.rev + v);
-    if (h >= n || ex <= 0) return UNVIS;
+    if (h >= n || ex <= 0) return;
     // a node with residual to the sink has label 1: the seeds' label is never
     // lowered, and a relabel of such a node gives 1 again
     int32_t t = h == 1u ? ldcg(g.term + v) : 0;
-    uint32_t next = UNVIS;
     const int nb[4] = {nb4.x, nb4.y, nb4.z, nb4.w};
     uint32_t r[4] = {r4.x, r4.y, r4.z, r4.w};
     uint32_t hn[4];
@@ -1406,20 +1407,15 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
             const uint32_t rk = (rv >> (2 * k)) & 3u;
             left[k] = atomicSub(g.res + (size_t)v * 4u + k, d);
             atomicAdd(g.res + (size_t)nb[k] * 4u + rk, d);
-            if (kAgg) {
-                // lanes pushing to the same neighbour now add their amounts in
-                // one atomic, issued by the group's first lane, which takes
-                // ownership when the neighbour's excess was zero
-                const cg::coalesced_group active = cg::coalesced_threads();
-                const cg::coalesced_group same = cg::labeled_partition(active, (unsigned)nb[k]);
-                const unsigned long long sum = cg::reduce(same, (unsigned long long)d,
-                                                          cg::plus<unsigned long long>());
-                if (same.thread_rank() == 0)
-                    o[k] = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb[k]), sum);
-            } else {
-                o[k] = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb[k]),
-                                 (unsigned long long)d);
-            }
+            // lanes pushing to the same neighbour now add their amounts in
+            // one atomic, issued by the group's first lane, which takes
+            // ownership when the neighbour's excess was zero
+            const cg::coalesced_group active = cg::coalesced_threads();
+            const cg::coalesced_group same = cg::labeled_partition(active, (unsigned)nb[k]);
+            const unsigned long long sum = cg::reduce(same, (unsigned long long)d,
+                                                      cg::plus<unsigned long long>());
+            if (same.thread_rank() == 0)
+                o[k] = atomicAdd(reinterpret_cast<unsigned long long*>(g.excess + nb[k]), sum);
         }
         // others only ever raise v's residuals meanwhile
         if (left[0] < r[0] || left[1] < r[1] || left[2] < r[2] || left[3] < r[3])
@@ -1446,19 +1442,15 @@ __device__ __forceinline__ uint32_t discharge_node(const SolveView& g, uint32_t 
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (o[k] != 0ull) continue;   // not the push that took ownership
-            if (may_chain && next == UNVIS) next = (uint32_t)nb[k];
-            else stage_push(g, st, (uint32_t)nb[k]);
+            if (o[k] == 0ull) stage_push(g, st, (uint32_t)nb[k]);   // the push that took ownership
         }
         if (fin) break;
     }
     const long long now = pushed ? (long long)self - pushed : ex;
     if (now > 0 && h < n) stage_push(g, st, v);   // keeps ownership
-    return next;
 }
 
-// discharge_node for a whole warp, a node per lane, without chaining or warp
-// aggregation: the lanes stay together, and the warp appends what they own with
+// discharge_node for a whole warp, a node per lane, without aggregation: the lanes stay together, and the warp appends what they own with
 // one shared atomic instead of one a node (long lists).
 __device__ __forceinline__ void discharge_warp(const SolveView& g, bool valid, uint32_t v, const Stage& st,
                                                Work& w)
@@ -1689,23 +1681,20 @@ __device__ __forceinline__ void discharge_quad(const SolveView& g, bool valid, u
 // became or stayed active; the block owns them), and append what the last
 // level left to the next active queue.  The stage is two halves of
 // stage_cap / 2 entries, ping-pong; entries that overflow a half go straight to
-// the queue.  With chains the round has one level.  `first` is the thread's
-// first entry (prefetch_entry).
+// the queue; a round of one level stages in the whole buffer.
 template <bool kAgg, bool kLean>
 __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t round, uint32_t cnt,
-                                               uint32_t first, uint32_t* s_buf, uint32_t stage_cap,
-                                               uint32_t* s_m, Work& w)
+                                               uint32_t* s_buf, uint32_t stage_cap, uint32_t* s_m,
+                                               Work& w)
 {
     Ctl* ctl = g.ctl;
     const uint32_t* in = (round & 1) ? g.act[1] : g.act[0];
     uint32_t* out = (round & 1) ? g.act[0] : g.act[1];
     uint32_t* gcnt = &ctl->act_cnt[(round + 1) % 3];
     const bool narrow = cnt <= g.chain_max_active;
-    const int hops = kLean ? 1 : narrow ? g.chain_hops : 1;
     const int levels = narrow ? g.dis_levels : g.dis_levels_wide;
-    const uint32_t half = stage_cap / 2u;
-    const bool warps = kLean || (!kAgg && hops <= 1 && levels > 1);
-    const bool quads = warps && cnt <= SPREAD_MAX;
+    const uint32_t half = kLean || levels > 1 ? stage_cap / 2u : stage_cap;
+    const bool quads = cnt <= SPREAD_MAX;
     const uint32_t per_pass = gridDim.x * (quads ? DTPB / 4u : (uint32_t)DTPB);
     for (uint32_t it = 0; it * per_pass < cnt; ++it) {
         uint32_t* cur = s_buf;
@@ -1717,7 +1706,7 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
             const uint32_t v = valid ? __ldcg(in + i) : 0u;
             if (valid && v >= g.n) raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
             if (__any_sync(0xffffffffu, valid)) discharge_quad(g, valid && v < g.n, v, st0, w);
-        } else if (warps) {
+        } else if (!kAgg) {
             const uint32_t i = queue_index(it, cnt);
             const bool valid = i < cnt;
             const uint32_t v = valid ? __ldcg(in + i) : 0u;
@@ -1726,15 +1715,9 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
         } else {
             const uint32_t i = queue_index(it, cnt);
             if (i < cnt) {
-                uint32_t v = (it == 0 && cnt <= SPREAD_MAX) ? first : __ldcg(in + i);
-                if (v < g.n) {
-                    for (int hop = 1;; ++hop) {
-                        v = discharge_node<kAgg>(g, v, st0, hop < hops, w);
-                        if (v == UNVIS) break;
-                    }
-                } else {
-                    raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
-                }
+                const uint32_t v = __ldcg(in + i);
+                if (v < g.n) discharge_node(g, v, st0, w);
+                else raise_error(ctl, (int)GPUPR_ERR_INVARIANT);
             }
         }
         __syncthreads();
@@ -1746,20 +1729,20 @@ __device__ __forceinline__ void discharge_body(const SolveView& g, uint32_t roun
             // the slot after next was read before the last block barrier
             if (threadIdx.x == 0) s_m[SUB + (nx == 2u ? 0u : nx + 1u)] = 0u;
             const Stage st{nxt, &s_m[SUB + nx], half, gcnt, out};
-            if (!kAgg && c <= QUAD_MAX) {
+            if (c <= QUAD_MAX) {
                 // a warp without a node has nothing to do
                 for (uint32_t j0 = (threadIdx.x >> 5) * 8u; j0 < c; j0 += DTPB / 4u) {
                     const uint32_t j = j0 + ((threadIdx.x & 31u) >> 2);
                     const bool valid = j < c;
                     discharge_quad(g, valid, valid ? cur[j] : 0u, st, w);
                 }
-            } else if (warps) {
+            } else if (!kAgg) {
                 for (uint32_t j0 = threadIdx.x & ~31u; j0 < c; j0 += DTPB) {
                     const uint32_t j = j0 + (threadIdx.x & 31u);
                     discharge_warp(g, j < c, j < c ? cur[j] : 0u, st, w);
                 }
             } else {
-                for (uint32_t j = threadIdx.x; j < c; j += DTPB) discharge_node<kAgg>(g, cur[j], st, false, w);
+                for (uint32_t j = threadIdx.x; j < c; j += DTPB) discharge_node(g, cur[j], st, w);
             }
             __syncthreads();
             uint32_t* tmp = cur;
@@ -1800,7 +1783,6 @@ __global__ void __launch_bounds__(DTPB) k_discharge(SolveView g, uint32_t round)
     __shared__ uint32_t s_m[16];
     __shared__ unsigned long long s_red[DTPB / 32];
     Ctl* ctl = g.ctl;
-    const uint32_t first = prefetch_entry((round & 1) ? g.act[1] : g.act[0], g.n);
     const uint32_t cnt = min(ldcg(&ctl->act_cnt[round % 3]), g.n);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         ctl->act_cnt[(round + 2) % 3] = 0u;
@@ -1810,7 +1792,7 @@ __global__ void __launch_bounds__(DTPB) k_discharge(SolveView g, uint32_t round)
     Work w;
     if (threadIdx.x < 16) s_m[threadIdx.x] = 0u;
     __syncthreads();
-    discharge_body<false, false>(g, round, cnt, first, s_buf, DTPB * 5, s_m, w);
+    discharge_body<false, false>(g, round, cnt, s_buf, DTPB * 5, s_m, w);
     reduce_work(ctl, w, 0u, s_red);
 }
 
@@ -1848,6 +1830,7 @@ struct PersistParams {
     unsigned long long budget;      // node visits per discharge phase, 0 = none
     unsigned long long limit_ns;    // solve time limit
     unsigned long long wait_ns;     // bound of one barrier wait
+    uint32_t relabel_min_rounds;    // least rounds of a phase (and of each extension)
     uint32_t relabel_rounds;        // rounds per discharge phase, 0 = none
 };
 
@@ -2118,7 +2101,6 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
             unsigned long long visits = 0;
             unsigned long long budget = p.budget;
             for (;;) {
-                const uint32_t first = prefetch_entry((r & 1) ? g.act[1] : g.act[0], g.n);
                 const uint32_t cnt = min(vload(&ctl->act_cnt[r % 3]), g.n);
                 if (cnt == 0) break;
                 if (rounds_total >= p.max_rounds) {
@@ -2128,14 +2110,14 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                 }
                 if (lead) ctl->act_cnt[(r + 2) % 3] = 0u;
                 if (lead) s_dr_t0 = gtimer();   // shared: keeps the discharge's registers free
-                discharge_body<kAgg, kLean>(g, r, cnt, first, s_buf, DTPB * 8, s_m, w);
+                discharge_body<kAgg, kLean>(g, r, cnt, s_buf, DTPB * 8, s_m, w);
                 if (lead) {
                     if (r == 0u) {
                         s_win_cnt = cnt;
                         s_win_r = 0u;
                     }
                     const unsigned long long t = gtimer();
-                    if (t > s_dr_limit && r + 1u >= s_win_r + RELABEL_MIN_ROUNDS) {
+                    if (t > s_dr_limit && r + 1u >= s_win_r + p.relabel_min_rounds) {
                         if ((float)cnt * RELABEL_GAIN <= (float)s_win_cnt) {
                             s_win_cnt = cnt;
                             s_win_r = r + 1u;
@@ -2365,17 +2347,17 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     const bool agg = opt.discharge_warp_aggregate > 0;
     TuneEntry te;
     const bool tuned = tune_lookup(g.n, &te);
-    // Discharge rounds run in block sub-levels; chains (a thread going on from
-    // node to node) are an option and replace the sub-levels of the rounds
-    // they apply to.  A caller's small round limit or relabel period counts
-    // rounds of one discharge per queued node, so it turns the sub-levels off
-    // (a sub-level round does the work of up to 16; 16384 rounds are far above
-    // what any of the graphs measured needs, at most 3,200 single ones, and 64
-    // sub-level rounds are as much as the default period of 1024 single ones).
+    // How far excess may travel in a round: 16 sub-levels, or as many as the
+    // caller's or a tuned entry's chain_hops where that is more.  A caller's
+    // small round limit or relabel period counts rounds of less: those run
+    // chain_hops sub-levels (default 4) when short and one when wide (16384
+    // rounds are far above what any of the graphs measured needs, at most 3,200
+    // of these, and 64 rounds of 16 are as much as the default period of 1024
+    // single ones).  Sub-levels took the place of a thread going on from node to
+    // node: a 2M-node integer graph at 4 hops 10.0 ms that way, 4.8 in sub-levels.
     const bool plain_rounds = opt.max_rounds < 16384ull || (opt.period > 0 && opt.period < 64);
-    const int chain_hops = opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : plain_rounds ? 4 : 1;
-    const bool lean = !agg && g.inm && !g.bottom_up && opt.bfs_tail_max <= 0 && opt.bfs_block_levels != 1 &&
-                      chain_hops <= 1 && !plain_rounds;
+    const int chain_hops = std::min(64, opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : plain_rounds ? 4 : 1);
+    const bool lean = !agg && g.inm && !g.bottom_up && opt.bfs_tail_max <= 0 && opt.bfs_block_levels != 1;
     const void* kern = g.arcm ? (agg ? (const void*)k_solve_persistent<true, true, false>
                                      : (const void*)k_solve_persistent<false, true, false>)
                        : agg  ? (const void*)k_solve_persistent<true, false, false>
@@ -2387,17 +2369,17 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     if (bps < 1) throw Error{GPUPR_ERR_CUDA, "persistent solver kernel cannot be resident"};
     // resident blocks per SM: a step of a small graph is one chain of
     // dependent L2 round trips plus a grid barrier whose cost grows with the
-    // number of blocks, while a large graph needs the threads to cover its
-    // frontiers and its blocks' BFS sub-levels.  Measured on B200 with the
-    // default BFS steps (15 graphs of 0.24-7.4M free nodes, three generators
-    // and the config-1 Delaunay proxy, median of 7): 2 is best or within 3%
-    // below 1.5M free nodes, 3 up to ~5M, 4 above (config 1: 3.3 ms at 2,
-    // 1.20 at 3; a 5.6M-node torus 5.07 at 3, 4.87 at 4).
+    // number of blocks, while a larger graph needs the threads to cover its
+    // frontiers and its blocks' sub-levels.  2 / 3 / 4 blocks
+    // (median of 7 solves, mean of three seeds, ms): a 60k-tet torus
+    // 0.385 / 0.390 / 0.398, a 120k-tet knot 0.695 / 0.724 / 0.740, a 220k-tet
+    // knot 0.484 / 0.473 / 0.485, a 450k-tet sphere 0.738 / 0.697 / 0.705, a
+    // 1M-tet torus 2.09 / 1.52 / 1.41, a 1.6M-tet sphere 2.0 / 1.3 / 1.2, a
+    // 2.4M-node integer graph 3.44 / 3.18 / 3.21, 11.7M nodes 8.3 / 7.4 / 6.5.
     // An autotuned entry for this size class replaces the rule.
     const int want = opt.blocks_per_sm > 0 ? opt.blocks_per_sm
                      : tuned                ? te.blocks_per_sm
-                     : g.n < 1500000u       ? 2
-                     : g.n < 5000000u       ? 3
+                     : g.n < 200000u        ? 2
                                             : 4;
     int used = want < bps ? want : bps;
     if (opt.max_blocks_per_sm > 0 && used > opt.max_blocks_per_sm) used = opt.max_blocks_per_sm;
@@ -2411,6 +2393,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     // cap the work rule normally reaches first.  The result does not depend on this
     // schedule: the solve always ends with an exact relabel.
     p.relabel_rounds = (uint32_t)(opt.period > 0 ? opt.period : 0);
+    p.relabel_min_rounds = plain_rounds ? RELABEL_MIN_ROUNDS_SINGLE : RELABEL_MIN_ROUNDS;
     const double wf = opt.work_factor > 0 ? opt.work_factor
                       : tuned                ? te.work_factor
                       : g.n < 500000u        ? 2.0
@@ -2427,8 +2410,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     GPUPR_CUDA(cudaMemsetAsync(g.ctl, 0, sizeof(Ctl), s));
     GPUPR_CUDA(cudaEventRecord(e0, s));
     SolveView gv = g;
-    gv.chain_hops = chain_hops;
-    gv.dis_levels = plain_rounds ? 1 : gv.chain_hops > 1 ? 1 : DIS_LEVELS;
+    gv.dis_levels = plain_rounds ? chain_hops : std::max(chain_hops, DIS_LEVELS);
     gv.dis_levels_wide = plain_rounds ? 1 : DIS_LEVELS_WIDE;
     gv.bfs_hops = opt.bfs_chain_hops > 0 ? std::min(opt.bfs_chain_hops, 64) : BFS_CHAIN_HOPS;
     // BFS steps expand BFS_BLOCK_LEVELS levels per block by default (measured
@@ -2468,7 +2450,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     out.engine = 2;
     out.blocks_per_sm = used;
     out.work_factor = wf;
-    out.chain_hops = gv.chain_hops;
+    out.chain_hops = chain_hops;
     out.chain_max_active = (int)gv.chain_max_active;
     out.launches = 1;
     out.raw_flow = (int64_t)hc.sink_flow;
