@@ -89,7 +89,7 @@ typedef struct {
     int64_t engine;             /* 1 one launch per step, 2 persistent */
     int64_t solve_blocks_per_sm;/* persistent engine: resident blocks per SM used */
     double relabel_work_factor; /* persistent engine: relabel work factor used */
-    int64_t chain_hops;         /* persistent engine: chained discharge used */
+    int64_t chain_hops;         /* persistent engine: short rounds (see the options) */
     int64_t chain_max_active;
     double sweep_ms;            /* persistent engine: active sweeps after each relabel
                                    (part of bfs_ms) */
@@ -126,16 +126,15 @@ typedef struct {
     int32_t bfs_batch;            /* BFS levels enqueued per host check, default 48 */
     int32_t block_size;           /* threads per block, default 256 */
     int32_t blocks_per_sm;        /* resident blocks per SM; default: 4 (one
-                                     launch per step), by graph size 2..4
-                                     (persistent: 2 below 1.5M free nodes, 3
-                                     below 5M, else 4) */
+                                     launch per step); persistent: 2 below
+                                     200,000 free nodes, else 4 */
     double work_relabel_factor;   /* relabel after this many node visits per
                                      free node since the last one; default 3
                                      (one launch per step); persistent: 2 below
                                      500k free nodes, 1 below 10M, else 0.5, and
                                      earlier once a discharge phase has taken
                                      0.9 times the relabel before it without
-                                     halving its active nodes */
+                                     losing a third of its active nodes */
     int32_t engine;               /* 0 auto (persistent when the device supports
                                      cooperative launch), 1 one launch per BFS
                                      level / round, 2 persistent */
@@ -512,13 +511,13 @@ gpupr_status gpupr_sample_tet_labels(const gpupr_brick_grid* grid, const double*
 
 /*
  * Autotuner (no counterpart in the reference).  The persistent engine's free
- * choices -- resident blocks per SM, the relabel work factor and chained
- * discharge -- change the time of a solve, never its result.  gpupr_autotune
+ * choices -- resident blocks per SM, the relabel work factor and the line
+ * between short and wide discharge rounds -- change the time of a solve, never its result.  gpupr_autotune
  * builds the reduced graph of the given cut once, then times the solve
  * (restoring the graph each time), `reps` times each (default 3),
  * interleaved: first every pair of blocks per SM {1,2,3,4} and work factor
- * {0.25,0.5,1,2}, then, with the best pair, chaining off, 4 hops up to 4096 or
- * 32768 active nodes, 8 hops up to 131072, beside the built-in rule.  The
+ * {0.25,0.5,1,2}, then, with the best pair, short rounds of up to 1, 4096, 32768
+ * or 131072 active nodes, beside the built-in rule.  The
  * setting with the lowest median (the rule's own values when it wins) is
  * kept for the graph's size class (free nodes in [2^k, 2^(k+1))).  Later solves whose options leave those fields at 0 use
  * the table; classes without an entry keep the built-in size rule.  The
@@ -531,7 +530,7 @@ typedef struct {
     double work_relabel_factor;
     double solve_ms;              /* median solve time of the chosen setting */
     double default_ms;            /* median solve time under the built-in rule */
-    int32_t chain_hops;           /* chained discharge (see gpupr_solve_options) */
+    int32_t chain_hops;           /* short rounds (see gpupr_solve_options) */
     int32_t chain_max_active;
 } gpupr_tune_entry;
 

@@ -1202,12 +1202,15 @@ constexpr uint32_t DIS_NARROW_MAX = 131072u;
 // 17.0 / 15.9 / 16.5 / 16.8, 80M-tet knot 68.5 / 66.6 / 68.7 / 69.4-73 / 77,
 // 12M-node integer graph 8.2 / 6.8 / 6.6 / 6.5 / 6.1.  Gains of 2 / 1.5 / 1.25:
 // a 2.4M-node integer graph 4.4 / 3.0 / 3.1 ms, a 5M-node one 5.1 / 4.6 / 4.5, the
-// 3.2M-tet sphere 2.7 / 2.9 / 3.2, a 2.6M-tet box 15.4 / 15.6 / 17.9, equal within
-// the spread of a variant's own runs over 32 graphs.  Where the caller's limits count
+// 3.2M-tet sphere 2.7 / 2.9 / 3.2, a 2.6M-tet box 15.4 / 15.6 / 17.9, 64 graphs of
+// 50k-4M tets 47.6 / 49.4 / 51.2, the 80M-tet knot 65.7 / 70 / 72-78: 1.5 up to 16M
+// nodes, 2 above.  Where the caller's limits count
 // smaller rounds (plain_rounds below), the least number is RELABEL_MIN_ROUNDS_SINGLE: a
 // graph that needs no second relabel is done by then.
 constexpr float RELABEL_TIME_RATIO = 0.9f;
 constexpr float RELABEL_GAIN = 1.5f;
+constexpr float RELABEL_GAIN_LARGE = 2.0f;
+constexpr uint32_t RELABEL_LARGE_MIN = 16000000u;
 constexpr uint32_t RELABEL_MIN_ROUNDS = 3u;
 constexpr uint32_t RELABEL_MIN_ROUNDS_SINGLE = 256u;
 
@@ -1830,6 +1833,7 @@ struct PersistParams {
     unsigned long long budget;      // node visits per discharge phase, 0 = none
     unsigned long long limit_ns;    // solve time limit
     unsigned long long wait_ns;     // bound of one barrier wait
+    float relabel_gain;             // the fall of the active nodes that extends a phase
     uint32_t relabel_min_rounds;    // least rounds of a phase (and of each extension)
     uint32_t relabel_rounds;        // rounds per discharge phase, 0 = none
 };
@@ -2118,7 +2122,7 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                     }
                     const unsigned long long t = gtimer();
                     if (t > s_dr_limit && r + 1u >= s_win_r + p.relabel_min_rounds) {
-                        if ((float)cnt * RELABEL_GAIN <= (float)s_win_cnt) {
+                        if ((float)cnt * p.relabel_gain <= (float)s_win_cnt) {
                             s_win_cnt = cnt;
                             s_win_r = r + 1u;
                             s_dr_limit = t + s_win;
@@ -2393,6 +2397,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     // cap the work rule normally reaches first.  The result does not depend on this
     // schedule: the solve always ends with an exact relabel.
     p.relabel_rounds = (uint32_t)(opt.period > 0 ? opt.period : 0);
+    p.relabel_gain = g.n < RELABEL_LARGE_MIN ? RELABEL_GAIN : RELABEL_GAIN_LARGE;
     p.relabel_min_rounds = plain_rounds ? RELABEL_MIN_ROUNDS_SINGLE : RELABEL_MIN_ROUNDS;
     const double wf = opt.work_factor > 0 ? opt.work_factor
                       : tuned                ? te.work_factor
