@@ -1592,10 +1592,16 @@ __device__ __forceinline__ void discharge_quad(const SolveView& g, bool valid, u
         r = ldcg(g.res + (size_t)v * 4u + k);
         rv = __ldg(g.rev + v);
     }
+    // one lane's values decide for the four: others add to the excess meanwhile,
+    // and lanes that split different amounts would push other than is released
+    const int first = (int)(threadIdx.x & 28u);
+    h = __shfl_sync(0xffffffffu, h, first);
+    ex = __shfl_sync(0xffffffffu, ex, first);
     bool live = h < n && ex > 0;
     if (live && nb >= 0) hn = ldcg(g.height + nb);
     int32_t t = 0;
     if (live && h == 1u) t = ldcg(g.term + v);
+    t = __shfl_sync(0xffffffffu, t, first);
     if (nb < 0) r = 0u;
     if (live && lead) ++w.visits;
     const uint32_t h0 = h;
