@@ -5,10 +5,11 @@
 // cudaMemcpyAsync from pageable memory goes through the driver's own staging
 // at the speed of one host thread.  Here a copy is cut into 1 MiB pieces that
 // rotate through a ring of pinned buffers: the calling thread and a small pool
-// of host threads each take the next piece, copy it between the caller's
-// array and its buffer and issue its DMA, so host copies and DMA overlap and the
-// copy runs near the PCIe rate.  The threads are woken once per copy, one waking
-// the next, and the caller starts at once: waking all of them for every 8 MiB
+// of host threads each take the next piece and copy it between the caller's
+// array and its buffer, and the calling thread issues the DMAs between its own
+// pieces, so host copies and DMA overlap and the copy runs near the PCIe rate.
+// The threads are woken once per copy, one waking the next, and the caller
+// starts at once: waking all of them for every 8 MiB
 // chunk, and waiting for the slowest of them at its end, cost more than the
 // copy itself up to tens of MB (13 MB: 1.63 -> 0.6-0.8 ms, 34 MB: 1.82 -> 1.4-1.6, the
 // driver's own path 0.67 and 1.74; 102 MB 3.6 -> 3.4-3.9).  Pinned
@@ -39,10 +40,51 @@ constexpr size_t kPiece = 1u << 20;     // bytes per staging buffer
 constexpr int kSlots = 32;              // staging buffers per set
 constexpr size_t kDirect = 1u << 20;    // below this, the driver's own path
 
-// A fixed set of host worker threads that run the parts of one job in
-// parallel; the calling thread takes parts too.  Each job is its own object
-// that workers pick up under the pool mutex, so a worker can never take a part
-// of a later job by mistake.
+// A copy's pieces, shared by its caller and the host threads that help it.  A
+// helper works on host memory only: it takes the next piece, waits until its
+// buffer is open, copies between the buffer and the caller's array and marks
+// the piece done.  It makes no CUDA call: a stream handle may mean another
+// stream in another thread (cudaStreamPerThread does), and the context current
+// in the caller need not be the one a helper would get.
+struct CopyJob {
+    const std::function<void(char*, size_t, size_t)>* fill = nullptr;   // alive while a piece is taken
+    char* pin = nullptr;
+    int64_t parts = 0;
+    size_t bytes = 0;
+    std::atomic<int64_t> next{0};       // the next piece to take
+    std::atomic<int64_t> open{0};       // pieces below it may be worked on
+    std::atomic<int64_t> finished{0};   // pieces taken and worked on (or skipped)
+    std::atomic<bool> stop{false};      // after an error: nothing more is copied
+    std::atomic<int64_t> done[kSlots];  // p + 1 of the last piece done in a buffer
+
+    CopyJob()
+    {
+        for (auto& d : done) d.store(0, std::memory_order_relaxed);
+    }
+    char* buffer(int64_t p) const { return pin + (size_t)(p % kSlots) * kPiece; }
+    size_t offset(int64_t p) const { return (size_t)p * kPiece; }
+    size_t length(int64_t p) const { return std::min(kPiece, bytes - offset(p)); }
+    void finish(int64_t p)
+    {
+        done[p % kSlots].store(p + 1, std::memory_order_release);
+        finished.fetch_add(1, std::memory_order_release);
+    }
+    void help()
+    {
+        for (;;) {
+            const int64_t p = next.fetch_add(1);
+            if (p >= parts) return;
+            while (open.load(std::memory_order_acquire) <= p && !stop.load(std::memory_order_relaxed))
+                std::this_thread::yield();
+            if (!stop.load(std::memory_order_relaxed)) (*fill)(buffer(p), offset(p), length(p));
+            finish(p);
+        }
+    }
+};
+
+// A fixed set of host worker threads that help the callers of copies.  Each
+// job is its own object that workers pick up under the pool mutex, so a worker
+// can never take a piece of a later job by mistake.
 class CopyPool {
 public:
     CopyPool()
@@ -64,55 +106,27 @@ public:
         for (auto& t : workers_) t.join();
     }
 
-    // Runs fn(0..parts-1), each part once and in ascending order of start, on
-    // the calling thread and up to `helpers` workers; returns when every part is
-    // done.
-    void run(int64_t parts, int64_t helpers, const std::function<void(int64_t)>& fn)
+    // Sends up to `helpers` workers to the job; returns how many.
+    int64_t enlist(const std::shared_ptr<CopyJob>& job, int64_t helpers)
     {
-        const int64_t calls = std::min(std::min((int64_t)workers_.size(), helpers), parts - 1);
-        if (calls <= 0) {
-            for (int64_t p = 0; p < parts; ++p) fn(p);
-            return;
-        }
-        auto job = std::make_shared<Job>();
-        job->fn = &fn;
-        job->parts = parts;
-        job->left = parts;
+        const int64_t want = std::min(std::min((int64_t)workers_.size(), helpers), job->parts - 1);
+        if (want <= 0) return 0;
+        int64_t sent = 0;
         try {
             std::lock_guard<std::mutex> lk(mu_);
-            for (int64_t i = 0; i < calls; ++i) calls_.push_back(job);
+            for (; sent < want; ++sent) calls_.push_back(job);
         } catch (const std::bad_alloc&) {
-            // fewer helpers; the job must not be left to those it has by unwinding
+            // fewer helpers: the caller does what they do not
         }
         cv_.notify_one();   // that thread wakes the next
-        job->run();
-        std::unique_lock<std::mutex> lk(job->mu);
-        job->cv.wait(lk, [&] { return job->left == 0; });
+        return sent;
     }
 
 private:
-    struct Job {
-        const std::function<void(int64_t)>* fn = nullptr;   // alive while parts are left
-        int64_t parts = 0;
-        std::atomic<int64_t> next{0};
-        int64_t left = 0;
-        std::mutex mu;
-        std::condition_variable cv;
-        void run()
-        {
-            for (;;) {
-                const int64_t p = next.fetch_add(1);
-                if (p >= parts) return;
-                (*fn)(p);
-                std::lock_guard<std::mutex> lk(mu);
-                if (--left == 0) cv.notify_all();
-            }
-        }
-    };
     void work()
     {
         for (;;) {
-            std::shared_ptr<Job> job;
+            std::shared_ptr<CopyJob> job;
             bool more;
             {
                 std::unique_lock<std::mutex> lk(mu_);
@@ -123,14 +137,14 @@ private:
                 more = !calls_.empty();
             }
             if (more) cv_.notify_one();
-            job->run();
+            job->help();
         }
     }
 
     std::vector<std::thread> workers_;
     std::mutex mu_;
     std::condition_variable cv_;
-    std::deque<std::shared_ptr<Job>> calls_;   // one entry per thread a job may use
+    std::deque<std::shared_ptr<CopyJob>> calls_;   // one entry per thread a job may use
     bool stop_ = false;
 };
 
@@ -223,35 +237,81 @@ int64_t copy_helpers(size_t bytes)
     return bytes < (4u << 20) ? 0 : std::max<int64_t>(1, (int64_t)(bytes / (10u << 20)));
 }
 
-// Runs `pieces` pieces through a staging set, each by one host thread (the
-// caller's device current): piece p uses buffer p % kSlots, after piece p -
-// kSlots is through with it.  step(p, pin, ev) copies piece p and issues its
-// DMA.  The first CUDA error is thrown by the caller's thread once all pieces
-// have been taken.
-template <class Step>
-void run_pieces(Staging& st, int64_t pieces, int64_t helpers, const Step& step)
+// Issues the DMA of piece p's buffer to the device.
+cudaError_t send(Staging& st, int64_t p, void* d_dst, size_t len, cudaStream_t s)
 {
-    int dev = 0;
-    GPUPR_CUDA(cudaGetDevice(&dev));
-    std::atomic<int64_t> done[kSlots];   // pieces a buffer has served
-    for (auto& d : done) d.store(0, std::memory_order_relaxed);
-    std::atomic<int> err{(int)cudaSuccess};
-    copy_pool().run(pieces, helpers, [&](int64_t p) {
-        const int k = (int)(p % kSlots);
-        // pieces start in order, so an earlier one of this buffer is on its way
-        while (done[k].load(std::memory_order_acquire) != p / kSlots) std::this_thread::yield();
-        if (err.load(std::memory_order_relaxed) == (int)cudaSuccess) {
-            cudaError_t e = cudaSetDevice(dev);
-            if (e == cudaSuccess && st.pending[k]) {
-                e = cudaEventSynchronize(st.ev[k]);
-                if (e == cudaSuccess) st.pending[k] = false;
+    const int k = (int)(p % kSlots);
+    const cudaError_t e = cudaMemcpyAsync(d_dst, st.pin + (size_t)k * kPiece, len, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return e;
+    st.pending[k] = true;
+    return cudaEventRecord(st.ev[k], s);
+}
+
+// The caller works on a piece in this many bytes at a time, so that pieces its
+// helpers have done wait for their DMA no longer than that.
+constexpr size_t kCallerStep = 256u << 10;
+
+// Runs a copy of `bytes` bytes, in pieces of kPiece,
+// through a staging set: fill(pin, offset, length) copies between a buffer and
+// the caller's array, on this thread or a helper's, once the buffer's last DMA is
+// through; after(p) issues the DMA that follows piece p, in order of the pieces.
+// All CUDA calls are this thread's.  After an error nothing more is copied and,
+// once no helper works on the job, the error is thrown.
+template <class After>
+void run_pieces(Staging& st, size_t bytes, int64_t helpers,
+                const std::function<void(char*, size_t, size_t)>& fill, const After& after)
+{
+    auto job = std::make_shared<CopyJob>();
+    job->fill = &fill;
+    job->pin = st.pin;
+    job->bytes = bytes;
+    const int64_t parts = job->parts = (int64_t)((bytes + kPiece - 1) / kPiece);
+    cudaError_t err = cudaSuccess;
+    int64_t passed = 0;   // pieces whose after() ran
+    int64_t open = 0;     // job->open
+    const int64_t ahead = 1 + copy_pool().enlist(job, helpers);   // pieces asked for at once
+    auto pass = [&] {
+        while (err == cudaSuccess && passed < parts &&
+               job->done[passed % kSlots].load(std::memory_order_acquire) == passed + 1)
+            err = after(passed++);
+    };
+    // a buffer opens when its last DMA is through: waited for only when a piece
+    // in it is asked for, or may be next
+    auto admit = [&] {
+        const int64_t want = std::min(std::min(parts, passed + kSlots), job->next.load() + ahead);
+        while (err == cudaSuccess && open < want) {
+            const int k = (int)(open % kSlots);
+            if (st.pending[k]) {
+                err = cudaEventSynchronize(st.ev[k]);
+                if (err != cudaSuccess) return;
+                st.pending[k] = false;
             }
-            if (e == cudaSuccess) e = step(p, st.pin + (size_t)k * kPiece, k);
-            if (e != cudaSuccess) err.store((int)e, std::memory_order_relaxed);
+            job->open.store(++open, std::memory_order_release);
         }
-        done[k].fetch_add(1, std::memory_order_release);
-    });
-    GPUPR_CUDA((cudaError_t)err.load());
+    };
+    int64_t mine = -1;   // this thread's piece
+    while (err == cudaSuccess && passed < parts) {
+        pass();
+        admit();
+        if (mine < 0) mine = job->next.fetch_add(1);
+        if (mine >= open || mine >= parts) {   // taken by others, or its buffer is not open yet
+            std::this_thread::yield();
+            continue;
+        }
+        const size_t off = job->offset(mine), len = job->length(mine);
+        for (size_t b = 0; b < len && err == cudaSuccess; b += kCallerStep) {
+            fill(job->buffer(mine) + b, off + b, std::min(kCallerStep, len - b));
+            pass();
+        }
+        job->finish(mine);
+        mine = -1;
+    }
+    if (err == cudaSuccess) return;
+    // no helper may touch the caller's array or the buffers once this returns
+    job->stop.store(true);
+    const int64_t taken = std::min(parts, job->next.exchange(parts)) - (mine >= 0 && mine < parts ? 1 : 0);
+    while (job->finished.load(std::memory_order_acquire) < taken) std::this_thread::yield();
+    GPUPR_CUDA(err);
 }
 
 }  // namespace
@@ -267,14 +327,13 @@ void host_to_device(void* d_dst, const void* h_src, size_t bytes, cudaStream_t s
     Staging& st = *lease.st;
     const char* src = static_cast<const char*>(h_src);
     char* dst = static_cast<char*>(d_dst);
-    run_pieces(st, (int64_t)((bytes + kPiece - 1) / kPiece), copy_helpers(bytes), [&](int64_t p, char* pin, int k) {
-        const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
-        std::memcpy(pin, src + off, len);
-        const cudaError_t e = cudaMemcpyAsync(dst + off, pin, len, cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) return e;
-        st.pending[k] = true;
-        return cudaEventRecord(st.ev[k], s);
-    });
+    run_pieces(
+        st, bytes, copy_helpers(bytes),
+        [&](char* pin, size_t off, size_t len) { std::memcpy(pin, src + off, len); },
+        [&](int64_t p) {
+            const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
+            return send(st, p, dst + off, len, s);
+        });
 }
 
 void device_to_host(void* h_dst, const void* d_src, size_t bytes, cudaStream_t s)
@@ -300,14 +359,13 @@ void device_to_host(void* h_dst, const void* d_src, size_t bytes, cudaStream_t s
         st.pending[k] = true;
         return cudaEventRecord(st.ev[k], s);
     };
-    // a ring of DMAs ahead; a piece's thread waits for it (run_pieces), copies
-    // it out and issues the one that follows in its buffer
+    // a ring of DMAs ahead; once a piece is copied out, the one that follows in
+    // its buffer is issued
     for (int64_t p = 0; p < std::min<int64_t>(pieces, kSlots); ++p) GPUPR_CUDA(issue(p));
-    run_pieces(st, pieces, copy_helpers(bytes), [&](int64_t p, char* pin, int) {
-        const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
-        std::memcpy(dst + off, pin, len);
-        return p + kSlots < pieces ? issue(p + kSlots) : cudaSuccess;
-    });
+    run_pieces(
+        st, bytes, copy_helpers(bytes),
+        [&](char* pin, size_t off, size_t len) { std::memcpy(dst + off, pin, len); },
+        [&](int64_t p) { return p + kSlots < pieces ? issue(p + kSlots) : cudaSuccess; });
 }
 
 // Nx4 integer topology (int32 or int64 elements, any byte strides, e.g. a
@@ -326,31 +384,33 @@ void upload_topology(int32_t* d_out, const void* host, uint64_t rows, int64_t ro
     const char* base = static_cast<const char*>(host);
     StagingLease lease = staging(0);
     Staging& st = *lease.st;
-    const uint64_t per = kPiece / 16u;
+    char* dst = reinterpret_cast<char*>(d_out);
+    const size_t bytes = rows * 16u;
     // a strided gather costs several times a memcpy: a helper per piece
-    const int64_t pieces = (int64_t)((rows + per - 1) / per);
-    run_pieces(st, pieces, pieces, [&](int64_t p, char* pin, int k) {
-        const uint64_t r0 = (uint64_t)p * per, r1 = std::min(rows, r0 + per);
-        int32_t* out = reinterpret_cast<int32_t*>(pin);
-        for (uint64_t r = r0; r < r1; ++r) {
-            const char* row = base + (int64_t)r * row_stride;
-            int32_t* o = out + (r - r0) * 4u;
-            for (int j = 0; j < 4; ++j) {
-                const char* e = row + (int64_t)j * col_stride;
-                if (elem_bytes == 8) {
-                    int64_t v;
-                    std::memcpy(&v, e, 8);
-                    o[j] = (int32_t)(uint32_t)(uint64_t)v;
-                } else {
-                    std::memcpy(&o[j], e, 4);
+    run_pieces(
+        st, bytes, (int64_t)((bytes + kPiece - 1) / kPiece),
+        [&](char* pin, size_t off, size_t len) {   // multiples of a row's 16 bytes
+            int32_t* out = reinterpret_cast<int32_t*>(pin);
+            const uint64_t r0 = off / 16u, r1 = r0 + len / 16u;
+            for (uint64_t r = r0; r < r1; ++r) {
+                const char* row = base + (int64_t)r * row_stride;
+                int32_t* o = out + (r - r0) * 4u;
+                for (int j = 0; j < 4; ++j) {
+                    const char* e = row + (int64_t)j * col_stride;
+                    if (elem_bytes == 8) {
+                        int64_t v;
+                        std::memcpy(&v, e, 8);
+                        o[j] = (int32_t)(uint32_t)(uint64_t)v;
+                    } else {
+                        std::memcpy(&o[j], e, 4);
+                    }
                 }
             }
-        }
-        const cudaError_t e = cudaMemcpyAsync(d_out + r0 * 4u, pin, (r1 - r0) * 16u, cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) return e;
-        st.pending[k] = true;
-        return cudaEventRecord(st.ev[k], s);
-    });
+        },
+        [&](int64_t p) {
+            const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
+            return send(st, p, dst + off, len, s);
+        });
 }
 
 namespace {
