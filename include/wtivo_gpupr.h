@@ -520,7 +520,8 @@ gpupr_status gpupr_sample_tet_labels(const gpupr_brick_grid* grid, const double*
  * or 131072 active nodes, beside the built-in rule.  The
  * setting with the lowest median (the rule's own values when it wins) is
  * kept for the graph's size class (free nodes in [2^k, 2^(k+1))).  Later solves whose options leave those fields at 0 use
- * the table; classes without an entry keep the built-in size rule.  The
+ * the table; classes without an entry keep the built-in size rule, and so do the
+ * lengths of rounds that a small max_rounds or global_relabel_period counts.  The
  * table is per process; gpupr_tune_table / gpupr_tune_table_set read and
  * replace it (to keep it across runs).  Arguments as gpupr_graph_cut.
  */

@@ -1,0 +1,58 @@
+"""A tuned size class changes the time of a solve, never whether it fits the
+caller's limits: rounds that a small max_rounds or relabel period counts are as
+long with an entry as without one, for a single solve and for a batch."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import cached_graph, to_cuda
+
+pytestmark = pytest.mark.gpu
+LIMITS = [dict(max_rounds=16383), dict(global_relabel_period=63)]
+
+
+@pytest.fixture
+def entries(built):
+    """Entries for every size class, with a line and hops that no untuned solve uses."""
+    import gpupr_capi
+
+    old = gpupr_capi.tune_table(), gpupr_capi.batch_tune_table()
+
+    def put(hops):
+        t = [dict(size_class=k, blocks_per_sm=2, work_relabel_factor=1.0, solve_ms=1.0, default_ms=1.0,
+                  chain_hops=hops, chain_max_active=hops) for k in range(32)] if hops else []
+        gpupr_capi.set_tune_table(t)
+        gpupr_capi.set_batch_tune_table(t)
+
+    yield put
+    gpupr_capi.set_tune_table(old[0])
+    gpupr_capi.set_batch_tune_table(old[1])
+
+
+@pytest.mark.parametrize("limit", LIMITS)
+@pytest.mark.parametrize("batch", [False, True])
+def test_hops_under_limits(entries, limit, batch):
+    import gpupr_capi
+
+    graphs = [cached_graph("torus", 5, 60_000), cached_graph("box", 4, 60_000)]
+    toff, voff, V, T, Nb, L = gpupr_capi.pack_batch(graphs if batch else graphs[:1])
+    t, n = to_cuda(T, Nb)
+
+    def cut(**kw):
+        o = gpupr_capi.options(**limit, **kw)
+        if batch:
+            out, _, st = gpupr_capi.graph_cut_batch(toff, voff, V, t, n, L, 10.0, opts=o)
+        else:
+            out, st = gpupr_capi.graph_cut(V, t, n, L, 10.0, opts=o)
+        return np.asarray(out), (st["chain_hops"], st["chain_max_active"])
+
+    entries(0)
+    labels, short = cut()
+    assert short == (4, 131072)
+    for tuned in 1, 4, 8, 40:
+        entries(tuned)
+        out, short = cut()
+        assert short == (4, 131072) and np.array_equal(out, labels)
+        assert cut(chain_hops=7, chain_max_active=9)[1] == (7, 9)   # the caller's own count stands

@@ -430,8 +430,11 @@ gpupr_solve_options batch_options(const gpupr_solve_options* options, uint32_t G
     if (batch_tune_lookup(free_n / (G ? G : 1u), &e)) {
         o.blocks_per_sm = e.blocks_per_sm;
         o.work_relabel_factor = e.work_factor;
-        o.chain_hops = e.chain_hops;
-        o.chain_max_active = e.chain_max_active;
+        // rounds the caller's limits count stay as long as without an entry
+        if (!counts_plain_rounds(resolve_options(&o, 8, 1024, 2000000ull))) {
+            o.chain_hops = e.chain_hops;
+            o.chain_max_active = e.chain_max_active;
+        }
     }
     return o;
 }

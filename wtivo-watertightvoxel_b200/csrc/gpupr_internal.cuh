@@ -324,6 +324,9 @@ struct SolveOptions {
 
 SolveOptions resolve_options(const gpupr_solve_options* o, int local_steps_raw,
                              int period_raw, uint64_t max_rounds_raw);
+// The persistent engine's rounds under the caller's limits: a small max_rounds or
+// relabel period counts rounds of a few sub-levels, not of 16.
+bool counts_plain_rounds(const SolveOptions& opt);
 
 struct SolveWorkspace {
     DevBuf<long long> excess;

@@ -2331,6 +2331,11 @@ SolveOptions resolve_options(const gpupr_solve_options* o, int local_steps_raw, 
     return r;
 }
 
+bool counts_plain_rounds(const SolveOptions& opt)
+{
+    return opt.max_rounds < 16384ull || (opt.period > 0 && opt.period < 64);
+}
+
 int persistent_blocks_per_sm()
 {
     int bps = 0;
@@ -2366,8 +2371,10 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     // of these, and 64 rounds of 16 are as much as the default period of 1024
     // single ones).  Sub-levels took the place of a thread going on from node to
     // node: a 2M-node integer graph at 4 hops 10.0 ms that way, 4.8 in sub-levels.
-    const bool plain_rounds = opt.max_rounds < 16384ull || (opt.period > 0 && opt.period < 64);
-    const int chain_hops = std::min(64, opt.chain_hops > 0 ? opt.chain_hops : tuned ? te.chain_hops : plain_rounds ? 4 : 1);
+    // A tuned entry has no say there: how far a counted round goes decides whether
+    // a solve fits its limit, and the tuner times only the other kind.
+    const bool plain_rounds = counts_plain_rounds(opt);
+    const int chain_hops = std::min(64, opt.chain_hops > 0 ? opt.chain_hops : plain_rounds ? 4 : tuned ? te.chain_hops : 1);
     const bool lean = !agg && g.inm && !g.bottom_up && opt.bfs_tail_max <= 0 && opt.bfs_block_levels != 1;
     const void* kern = g.arcm ? (agg ? (const void*)k_solve_persistent<true, true, false>
                                      : (const void*)k_solve_persistent<false, true, false>)
@@ -2442,7 +2449,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
                   : opt.bfs_tail_max > 0 ? std::min<uint32_t>((uint32_t)opt.bfs_tail_max, TAIL_CAP)
                                          : BFS_TAIL_DEFAULT;
     gv.chain_max_active = opt.chain_max_active > 0 ? (uint32_t)opt.chain_max_active
-                          : tuned                  ? (uint32_t)te.chain_max_active
+                          : tuned && !plain_rounds ? (uint32_t)te.chain_max_active
                                                    : DIS_NARROW_MAX;
     void* args[] = {&gv, &p};
     GPUPR_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(DTPB), args, dsmem, s));
