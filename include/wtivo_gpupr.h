@@ -89,8 +89,8 @@ typedef struct {
     int64_t engine;             /* 1 one launch per step, 2 persistent */
     int64_t solve_blocks_per_sm;/* persistent engine: resident blocks per SM used */
     double relabel_work_factor; /* persistent engine: relabel work factor used */
-    int64_t chain_hops;         /* persistent engine: short rounds (see the options) */
-    int64_t chain_max_active;
+    int64_t chain_hops;         /* persistent engine: sub-levels of a short round */
+    int64_t chain_max_active;   /* ... and the most active nodes of one */
     double sweep_ms;            /* persistent engine: active sweeps after each relabel
                                    (part of bfs_ms) */
     uint64_t graphs_retired;    /* batch: graphs finished and left out of the
@@ -531,8 +531,8 @@ typedef struct {
     double work_relabel_factor;
     double solve_ms;              /* median solve time of the chosen setting */
     double default_ms;            /* median solve time under the built-in rule */
-    int32_t chain_hops;           /* short rounds (see gpupr_solve_options) */
-    int32_t chain_max_active;
+    int32_t chain_hops;           /* sub-levels of a short round (see gpupr_solve_options) */
+    int32_t chain_max_active;     /* the most active nodes of one */
 } gpupr_tune_entry;
 
 gpupr_status gpupr_autotune(const double* vertices, uint64_t n_vertices, int vertices_on_device,

@@ -56,3 +56,22 @@ def test_hops_under_limits(entries, limit, batch):
         out, short = cut()
         assert short == (4, 131072) and np.array_equal(out, labels)
         assert cut(chain_hops=7, chain_max_active=9)[1] == (7, 9)   # the caller's own count stands
+
+
+def test_stats_report_what_ran(entries):
+    """Short rounds run 16 sub-levels, or the hops asked for where that is more."""
+    import gpupr_capi
+
+    g = cached_graph("torus", 5, 60_000)
+    t, n = to_cuda(g["tets"], g["neighbors"])
+
+    def hops(**kw):
+        return gpupr_capi.graph_cut(g["vertices"], t, n, g["labels"], 10.0, opts=gpupr_capi.options(**kw))[1]["chain_hops"]
+
+    entries(0)
+    assert [hops(), hops(chain_hops=1), hops(chain_hops=16), hops(chain_hops=40)] == [16, 16, 16, 40]
+    entries(8)
+    assert [hops(), hops(chain_hops=40)] == [16, 40]
+    entries(0)
+    e = gpupr_capi.autotune(g["vertices"], t, n, g["labels"], 10.0, reps=1)
+    assert e["chain_hops"] == 16

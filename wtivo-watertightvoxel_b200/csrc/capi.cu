@@ -241,14 +241,14 @@ void run_graph_cut(const double* vertices, uint64_t nv, int v_dev, const int32_t
 // batch's segmented union): timed solves with the residuals and terminals
 // restored before each, every candidate `reps` times, interleaved so slow
 // drifts of the clock hit every candidate alike.  Stage 1: resident blocks per
-// SM x relabel work factor with the base chaining; stage 2: chaining with the
-// best pair.  Both stages also time `base` itself (the built-in rule), and the
+// SM x relabel work factor; stage 2: the line between short and wide rounds with
+// the best pair (hops up to the 16 sub-levels of a short round change nothing).  Both stages also time `base` itself (the built-in rule), and the
 // entry never replaces the rule by a setting that was not faster.  A
 // candidate's zero fields take base's values.
 struct TuneCand {
     int bps;
     double wf;
-    int hops, cmax;
+    int cmax;
     std::vector<double> ms;
     SolveResult last;   // settings the solve actually used
 };
@@ -277,7 +277,6 @@ TuneEntry two_stage_tune(ReducedGraph& g, const Segments* segs, const gpupr_solv
                 o.engine = 2;
                 if (c.bps) o.blocks_per_sm = c.bps;
                 if (c.wf > 0) o.work_relabel_factor = c.wf;
-                if (c.hops) o.chain_hops = c.hops;
                 if (c.cmax) o.chain_max_active = c.cmax;
                 SolveOptions opt = resolve_options(&o, local_steps, 1024, 2000000ull);
                 SolveResult sr;
@@ -287,17 +286,16 @@ TuneEntry two_stage_tune(ReducedGraph& g, const Segments* segs, const gpupr_solv
             }
     };
     std::vector<TuneCand> c1;
-    c1.push_back({0, 0.0, 0, 0, {}, {}});
+    c1.push_back({0, 0.0, 0, {}, {}});
     for (int bp : {1, 2, 3, 4})
-        for (double f : {0.25, 0.5, 1.0, 2.0}) c1.push_back({bp, f, 0, 0, {}, {}});
+        for (double f : {0.25, 0.5, 1.0, 2.0}) c1.push_back({bp, f, 0, {}, {}});
     run(c1);
     size_t bi = 1;
     for (size_t i = 2; i < c1.size(); ++i)
         if (median_of(c1[i].ms) < median_of(c1[bi].ms)) bi = i;
     std::vector<TuneCand> c2;
-    c2.push_back({0, 0.0, 0, 0, {}, {}});
-    for (auto hc : {std::pair<int, int>{1, 1}, {4, 4096}, {4, 32768}, {8, 131072}})
-        c2.push_back({c1[bi].bps, c1[bi].wf, hc.first, hc.second, {}, {}});
+    c2.push_back({0, 0.0, 0, {}, {}});
+    for (int line : {1, 4096, 32768, 131072}) c2.push_back({c1[bi].bps, c1[bi].wf, line, {}, {}});
     run(c2);
     size_t bj = 0;
     for (size_t i = 1; i < c2.size(); ++i)

@@ -370,7 +370,8 @@ struct SolveResult {
     int engine = 1;                // 1 one launch per step, 2 persistent
     int blocks_per_sm = 0;         // persistent engine: grid used
     double work_factor = 0.0;      // persistent engine: relabel work factor used
-    int chain_hops = 0, chain_max_active = 0;   // persistent engine: short rounds used
+    int chain_hops = 0, chain_max_active = 0;   // persistent engine: sub-levels of a short round, and
+                                                // the line to a wide one
     int relabel_tiles = 0;         // persistent engine: 1 = tiled relabels ran
     uint64_t tile_steps = 0, tile_procs = 0, tile_loads = 0, tile_writes = 0;
     uint64_t dround_cnt[3] = {0, 0, 0};  // discharge rounds by active nodes (<= 4096, <= 131072, larger)

@@ -2469,7 +2469,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     out.engine = 2;
     out.blocks_per_sm = used;
     out.work_factor = wf;
-    out.chain_hops = chain_hops;
+    out.chain_hops = gv.dis_levels;
     out.chain_max_active = (int)gv.chain_max_active;
     out.launches = 1;
     out.raw_flow = (int64_t)hc.sink_flow;
