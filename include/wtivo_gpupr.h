@@ -147,7 +147,8 @@ typedef struct {
                                      max_rounds below 16384 and a
                                      global_relabel_period of 1 to 63 count
                                      smaller rounds: chain_hops sub-levels
-                                     (default 4) short, one wide */
+                                     short (default 8 under max_rounds, 4
+                                     under a period), two and one wide */
     int32_t bfs_bottom_up;        /* persistent engine: 1 = direction-optimizing
                                      global relabels (bottom-up steps over the
                                      nodes the previous relabel reached and this

@@ -10,7 +10,7 @@ import torch
 from conftest import cached_graph, to_cuda
 
 pytestmark = pytest.mark.gpu
-LIMITS = [dict(max_rounds=16383), dict(global_relabel_period=63)]
+LIMITS = [(dict(max_rounds=16383), 8), (dict(global_relabel_period=63), 4), (dict(max_rounds=16383, global_relabel_period=63), 8)]
 
 
 @pytest.fixture
@@ -31,9 +31,9 @@ def entries(built):
     gpupr_capi.set_batch_tune_table(old[1])
 
 
-@pytest.mark.parametrize("limit", LIMITS)
+@pytest.mark.parametrize("limit,levels", LIMITS)
 @pytest.mark.parametrize("batch", [False, True])
-def test_hops_under_limits(entries, limit, batch):
+def test_hops_under_limits(entries, limit, levels, batch):
     import gpupr_capi
 
     graphs = [cached_graph("torus", 5, 60_000), cached_graph("box", 4, 60_000)]
@@ -50,11 +50,11 @@ def test_hops_under_limits(entries, limit, batch):
 
     entries(0)
     labels, short = cut()
-    assert short == (4, 131072)
+    assert short == (levels, 131072)
     for tuned in 1, 4, 8, 40:
         entries(tuned)
         out, short = cut()
-        assert short == (4, 131072) and np.array_equal(out, labels)
+        assert short == (levels, 131072) and np.array_equal(out, labels)
         assert cut(chain_hops=7, chain_max_active=9)[1] == (7, 9)   # the caller's own count stands
 
 
@@ -75,3 +75,14 @@ def test_stats_report_what_ran(entries):
     entries(0)
     e = gpupr_capi.autotune(g["vertices"], t, n, g["labels"], 10.0, reps=1)
     assert e["chain_hops"] == 16
+
+
+@pytest.mark.parametrize("seed", [5, 6, 7])
+def test_round_limits_that_held(built, seed):
+    """A solve fits the round limits it fitted with chains of hops (63-92 rounds on
+    these graphs; 207-265 with rounds of four sub-levels and 256 of them before a relabel)."""
+    from test_gpu_sublevels import check, grid_graph
+
+    g = grid_graph(200_000, np.random.default_rng(seed), 20, 50)
+    for _ in range(3):
+        assert check(*g, max_rounds=100)["rounds"] <= 100

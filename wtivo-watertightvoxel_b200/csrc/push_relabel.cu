@@ -1205,14 +1205,16 @@ constexpr uint32_t DIS_NARROW_MAX = 131072u;
 // 3.2M-tet sphere 2.7 / 2.9 / 3.2, a 2.6M-tet box 15.4 / 15.6 / 17.9, 64 graphs of
 // 50k-4M tets 47.6 / 49.4 / 51.2, the 80M-tet knot 65.7 / 70 / 72-78: 1.5 up to 16M
 // nodes, 2 above.  Where the caller's limits count
-// smaller rounds (plain_rounds below), the least number is RELABEL_MIN_ROUNDS_SINGLE: a
-// graph that needs no second relabel is done by then.
+// smaller rounds (plain_rounds below), the least number is as many as make the
+// same 48 hops: with 256 rounds, graphs with a few stuck nodes spent up to 512 of a
+// caller's rounds on them (60k-tet knots 512 rounds and 7.0 ms, with 6 rounds of
+// 8 levels 24-36 and 0.9 ms).
 constexpr float RELABEL_TIME_RATIO = 0.9f;
 constexpr float RELABEL_GAIN = 1.5f;
 constexpr float RELABEL_GAIN_LARGE = 2.0f;
 constexpr uint32_t RELABEL_LARGE_MIN = 16000000u;
 constexpr uint32_t RELABEL_MIN_ROUNDS = 3u;
-constexpr uint32_t RELABEL_MIN_ROUNDS_SINGLE = 256u;
+constexpr uint32_t RELABEL_MIN_HOPS = RELABEL_MIN_ROUNDS * (uint32_t)DIS_LEVELS;
 
 // Free nodes from which the persistent engine relabels by tiles by default.
 constexpr uint32_t RELABEL_TILES_DEFAULT_MIN = 0xFFFFFFFFu;
@@ -2331,9 +2333,12 @@ SolveOptions resolve_options(const gpupr_solve_options* o, int local_steps_raw, 
     return r;
 }
 
+// max_rounds below which a round limit counts smaller rounds (solve_persistent)
+constexpr uint64_t FEW_ROUNDS = 16384u;
+
 bool counts_plain_rounds(const SolveOptions& opt)
 {
-    return opt.max_rounds < 16384ull || (opt.period > 0 && opt.period < 64);
+    return opt.max_rounds < FEW_ROUNDS || (opt.period > 0 && opt.period < 64);
 }
 
 int persistent_blocks_per_sm()
@@ -2364,17 +2369,28 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     TuneEntry te;
     const bool tuned = tune_lookup(g.n, &te);
     // How far excess may travel in a round: 16 sub-levels, or as many as the
-    // caller's or a tuned entry's chain_hops where that is more.  A caller's
-    // small round limit or relabel period counts rounds of less: those run
-    // chain_hops sub-levels (default 4) when short and one when wide (16384
-    // rounds are far above what any of the graphs measured needs, at most 3,200
-    // of these, and 64 rounds of 16 are as much as the default period of 1024
-    // single ones).  Sub-levels took the place of a thread going on from node to
-    // node: a 2M-node integer graph at 4 hops 10.0 ms that way, 4.8 in sub-levels.
+    // caller's or a tuned entry's chain_hops where that is more.  Sub-levels took the
+    // place of a thread going on from node to node: a 2M-node integer graph at 4
+    // hops 10.0 ms that way, 4.8 in sub-levels.
+    // A caller's small round limit or relabel period counts rounds of less, about
+    // what a round was with such chains: chain_hops sub-levels when short, by
+    // default 8 (2 when wide) under a round limit and 4 (1) under a period.  (16384
+    // rounds are far above what any of the graphs measured needs, at most 3,200 of
+    // the small ones, and 64 rounds of 16 are as much as the default period of 1024
+    // single ones.)  With 8 and 2 a solve takes no more of them than it took chained
+    // rounds, nor longer, over 45 graphs of 5k-20M tets and nodes; with 4 and 1 up to
+    // seven times as many (50k nodes 74-586, chained 83-88) or always a few more (a
+    // 3M-tet sphere 277-294, chained 222-270, now 31-36), and then failed limits that
+    // it had kept.
     // A tuned entry has no say there: how far a counted round goes decides whether
     // a solve fits its limit, and the tuner times only the other kind.
     const bool plain_rounds = counts_plain_rounds(opt);
-    const int chain_hops = std::min(64, opt.chain_hops > 0 ? opt.chain_hops : plain_rounds ? 4 : tuned ? te.chain_hops : 1);
+    const bool few_rounds = opt.max_rounds < FEW_ROUNDS;
+    const int chain_hops = std::min(64, opt.chain_hops > 0 ? opt.chain_hops
+                                        : few_rounds       ? 8
+                                        : plain_rounds     ? 4
+                                        : tuned            ? te.chain_hops
+                                                           : 1);
     const bool lean = !agg && g.inm && !g.bottom_up && opt.bfs_tail_max <= 0 && opt.bfs_block_levels != 1;
     const void* kern = g.arcm ? (agg ? (const void*)k_solve_persistent<true, true, false>
                                      : (const void*)k_solve_persistent<false, true, false>)
@@ -2412,7 +2428,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     // schedule: the solve always ends with an exact relabel.
     p.relabel_rounds = (uint32_t)(opt.period > 0 ? opt.period : 0);
     p.relabel_gain = g.n < RELABEL_LARGE_MIN ? RELABEL_GAIN : RELABEL_GAIN_LARGE;
-    p.relabel_min_rounds = plain_rounds ? RELABEL_MIN_ROUNDS_SINGLE : RELABEL_MIN_ROUNDS;
+    p.relabel_min_rounds = plain_rounds ? (RELABEL_MIN_HOPS + chain_hops - 1u) / chain_hops : RELABEL_MIN_ROUNDS;
     const double wf = opt.work_factor > 0 ? opt.work_factor
                       : tuned                ? te.work_factor
                       : g.n < 500000u        ? 2.0
@@ -2430,7 +2446,7 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     GPUPR_CUDA(cudaEventRecord(e0, s));
     SolveView gv = g;
     gv.dis_levels = plain_rounds ? chain_hops : std::max(chain_hops, DIS_LEVELS);
-    gv.dis_levels_wide = plain_rounds ? 1 : DIS_LEVELS_WIDE;
+    gv.dis_levels_wide = few_rounds ? 2 : plain_rounds ? 1 : DIS_LEVELS_WIDE;
     gv.bfs_hops = opt.bfs_chain_hops > 0 ? std::min(opt.bfs_chain_hops, 64) : BFS_CHAIN_HOPS;
     // BFS steps expand BFS_BLOCK_LEVELS levels per block by default (measured
     // against per-thread chains of 4: benchmark graph 77.7 -> 68.0 ms, 8M-tet
