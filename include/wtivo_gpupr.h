@@ -134,7 +134,8 @@ typedef struct {
                                      500k free nodes, 1 below 10M, else 0.5, and
                                      earlier once a discharge phase has taken
                                      0.9 times the relabel before it without
-                                     losing a third of its active nodes */
+                                     losing a third of its active nodes (half
+                                     of them from 16M free nodes on) */
     int32_t engine;               /* 0 auto (persistent when the device supports
                                      cooperative launch), 1 one launch per BFS
                                      level / round, 2 persistent */

@@ -19,8 +19,9 @@
 //    expands the nodes it labelled itself for up to 16 levels from its
 //    shared-memory stage (or, as an option, a thread labels several nodes in
 //    a row), so one grid barrier covers several levels; reachability is
-//    exact in every case and labels converge to distances while lowered
-//    labels propagate.  The active queue is collected after each BFS by a
+//    exact in every case, and labels converge to distances where lowered
+//    labels propagate (graphs of 36.4M free nodes and more at four blocks an
+//    SM, bfs_step_levels_body).  The active queue is collected after each BFS by a
 //    streaming sweep, in node order (engine 1 appends it during its
 //    level-synchronous BFS, .cu:360-402 and :149-166).
 //  * Reverse slots are precomputed at build time (2 bits per slot), so a push
@@ -1072,7 +1073,10 @@ __device__ __forceinline__ void bfs_expand_quad(const SolveView& g, bool valid, 
 // nodes, and any that overflow a half, go to the next step's queue.  Labels
 // are corrected like the chained steps' (atomicMin, re-queued while
 // `propagate`): a node labelled here before another block reaches it by a
-// shorter path is lowered and expanded again.  Frontier entries may carry
+// shorter path is lowered and expanded again.  The caller allows that while the
+// step's worst case fits the queue, which below 36.4M free nodes (at four blocks
+// an SM) it never does: there a lowered label stays where it is, and labels are
+// lengths of paths but not always of shortest ones.  Frontier entries may carry
 // different labels: each expansion reads its node's label.
 template <bool kLean>
 __device__ __forceinline__ void bfs_step_levels_body(const SolveView& g, uint32_t L, uint32_t cnt,
@@ -1200,11 +1204,15 @@ constexpr uint32_t DIS_NARROW_MAX = 131072u;
 // of the rule, 6.7 ms with it).  Ratios of 0.6 / 0.8 / 0.9 / 1.2 / 1.6 (mean of
 // three seeds): 3.2M-tet sphere 2.9 / 3.1 / 3.3 / 3.9 / 4.7 ms, 8M-tet box 17.8 /
 // 17.0 / 15.9 / 16.5 / 16.8, 80M-tet knot 68.5 / 66.6 / 68.7 / 69.4-73 / 77,
-// 12M-node integer graph 8.2 / 6.8 / 6.6 / 6.5 / 6.1.  Gains of 2 / 1.5 / 1.25:
-// a 2.4M-node integer graph 4.4 / 3.0 / 3.1 ms, a 5M-node one 5.1 / 4.6 / 4.5, the
-// 3.2M-tet sphere 2.7 / 2.9 / 3.2, a 2.6M-tet box 15.4 / 15.6 / 17.9, 64 graphs of
-// 50k-4M tets 47.6 / 49.4 / 51.2, the 80M-tet knot 65.7 / 70 / 72-78: 1.5 up to 16M
-// nodes, 2 above.  Where the caller's limits count
+// 12M-node integer graph 8.2 / 6.8 / 6.6 / 6.5 / 6.1.  Gains of 1.5 / 2
+// (mean of three seeds, in tets or nodes): integer graphs of 2.4M 3.1 / 4.2 ms, 5M 4.6 /
+// 5.7, 8M 5.4 / 6.0, 11.7M 6.7 / 6.7; a 2.6M box 14.9 / 15.8, 10M torus 8.7 / 9.6,
+// 16M knot 12.3 / 14.3, 30M torus 24.4 / 26.0 against a 3.2M sphere 2.8 / 2.7, 8M knot
+// 7.2 / 6.8, 12M knot 11.1 / 9.6, 40M knot 33.1 / 30.9, 80M knot 72.7 / 70.1, 64
+// graphs of 50k-4M tets (56M in all) 49.4 / 47.6; equal on an 8M and a 20M box, a
+// 14M sphere, a 24M knot.  Size does not tell them apart sharply: below 16M nodes 2
+// costs more where it loses (a third on one) than it gives where it wins, above it
+// wins on the largest.  Where the caller's limits count
 // smaller rounds (plain_rounds below), the least number is as many as make the
 // same 48 hops: with 256 rounds, graphs with a few stuck nodes spent up to 512 of a
 // caller's rounds on them (60k-tet knots 512 rounds and 7.0 ms, with 6 rounds of
@@ -2420,11 +2428,12 @@ void solve_persistent(const SolveView& g, const SolveOptions& opt, cudaStream_t 
     const unsigned grid = (unsigned)(sm_count() * used);
     PersistParams p{};
     p.max_rounds = opt.max_rounds;
-    // Global relabels: a discharge phase ends once its node visits exceed
-    // work_factor x n (measured on B200: 2 suits graphs below ~500k free
-    // nodes, 1 up to ~10M, 0.5 above: 19M nodes 14.5 vs 16.6 ms, a 64-graph
-    // union of 50M 80.7 vs 89.8 ms), or after global_relabel_period rounds, a
-    // cap the work rule normally reaches first.  The result does not depend on this
+    // Global relabels: besides by time (RELABEL_TIME_RATIO), a discharge phase ends
+    // once its node visits exceed work_factor x n, or after global_relabel_period
+    // rounds.  The time rule comes first nearly always: without a limit on visits 21
+    // graphs of 2.4M-80M took within the spread of their runs of the same time (80M
+    // knot 70.1 -> 67.4 ms, 2.4M integer graph 3.1 -> 3.3).  The factors by size are
+    // those that suited one level a round.  The result does not depend on this
     // schedule: the solve always ends with an exact relabel.
     p.relabel_rounds = (uint32_t)(opt.period > 0 ? opt.period : 0);
     p.relabel_gain = g.n < RELABEL_LARGE_MIN ? RELABEL_GAIN : RELABEL_GAIN_LARGE;
