@@ -2046,7 +2046,11 @@ __global__ void __launch_bounds__(DTPB, 4) k_solve_persistent(SolveView g, Persi
                     bottom_up = cc != 0u && (float)rem <= g.bu_ratio * (float)cnt;
                 }
                 if (!kLean && !g.bottom_up && g.tail_max && cnt <= g.tail_max) {
-                    // a short frontier: block 0 runs the next levels alone
+                    // a short frontier: block 0 runs the next levels alone, once
+                    // every block has read this level's count and the last tail
+                    // step's level (it rewrites both; a block that came late
+                    // would leave the others' path)
+                    if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
                     if (blockIdx.x == 0) bfs_tail_body(g, L, cnt, s_buf, s_m, bfs_visits);
                     exact = false;
                     if (!(ok = grid_barrier(ctl, s_bar, p.wait_ns))) break;
