@@ -37,7 +37,7 @@ struct Op { void* dst; const void* src; size_t n; cudaEvent_t ev; };
 std::mutex mu;
 std::map<cudaStream_t, std::deque<Op>> queues;   // copies and events not carried out yet
 std::map<cudaEvent_t, cudaStream_t> waiting;     // the queue an event is in
-std::atomic<long> foreign{0}, calls{0}, fail_at{-1};
+std::atomic<long> foreign{0}, calls{0}, dmas{0}, fail_at{-1};
 thread_local bool caller = false;
 cudaError_t note()
 {
@@ -86,6 +86,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*)
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t s)
 {
     const cudaError_t e = note();
+    ++dmas;
     std::lock_guard<std::mutex> l(mu);
     if (e == cudaSuccess) queues[s].push_back({dst, src, n, nullptr});
     return e;
@@ -113,6 +114,8 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s)
     return e;
 }
 long fake_foreign() { return foreign.exchange(0); }
+long fake_calls() { return calls.exchange(0); }
+long fake_dmas() { return dmas.exchange(0); }
 void fake_fail_at(long n) { calls = 0; fail_at = n; }
 int fake_h2d(void* d, const void* h, size_t n, void* s)
 { return guarded([&] { gpupr::host_to_device(d, h, n, (cudaStream_t)s); }); }
@@ -140,7 +143,8 @@ def lib(tmp_path_factory):
     x.fake_topology.argtypes = [p, p, ctypes.c_uint64, i, i, ctypes.c_int, p]
     x.fake_sync.argtypes = [p]
     x.fake_fail_at.argtypes = [ctypes.c_long]
-    x.fake_foreign.restype = ctypes.c_long
+    for f in (x.fake_foreign, x.fake_calls, x.fake_dmas):
+        f.restype = ctypes.c_long
     return x
 
 
@@ -222,20 +226,38 @@ def test_threads(lib):
     assert ok == [True] * 18
 
 
-@pytest.mark.parametrize("at", [3, 4, 5, 9, 40, 41, 66, 90, 120, 150])
-def test_errors(lib, at):
+def test_errors(lib):
     """A CUDA error anywhere in a copy comes back as the call's error, no helper
     works on after it, and the next copy is whole."""
     src = data(70 * MB + 48, 1)
     dev = np.zeros_like(src)
     for f, d, s in ((lib.fake_h2d, dev, src), (lib.fake_d2h, dev, src)):
-        lib.fake_fail_at(at)
-        rc = f(d.ctypes.data, s.ctypes.data, s.size, 5)
-        lib.fake_fail_at(-1)
-        lib.fake_sync(5)
-        assert rc == 1
-        d[:] = 0
         assert f(d.ctypes.data, s.ctypes.data, s.size, 5) == 0
         lib.fake_sync(5)
-        assert np.array_equal(d, s)
-        d[:] = 0
+        lib.fake_calls()
+        assert f(d.ctypes.data, s.ctypes.data, s.size, 5) == 0
+        calls = lib.fake_calls()   # give or take which pieces share a DMA
+        lib.fake_sync(5)
+        for at in [2, 3, 4, 5, 6] + [calls * k // 10 for k in range(1, 9)]:
+            lib.fake_fail_at(at)
+            rc = f(d.ctypes.data, s.ctypes.data, s.size, 5)
+            lib.fake_fail_at(-1)
+            lib.fake_sync(5)
+            assert rc == 1, at
+            d[:] = 0
+            assert f(d.ctypes.data, s.ctypes.data, s.size, 5) == 0
+            lib.fake_sync(5)
+            assert np.array_equal(d, s)
+            d[:] = 0
+
+
+def test_pieces_share_a_dma(lib):
+    """Past its ends a large copy takes several pieces to a DMA."""
+    src = data(150 * MB + 3, 2)
+    dev = np.zeros_like(src)
+    lib.fake_dmas()
+    assert lib.fake_h2d(dev.ctypes.data, src.ctypes.data, src.size, 3) == 0
+    lib.fake_sync(3)
+    assert np.array_equal(dev, src) and lib.fake_dmas() < 151 // 2
+    assert lib.fake_d2h(src.ctypes.data, dev.ctypes.data, src.size, 3) == 0
+    assert np.array_equal(dev, src) and lib.fake_dmas() < 151 // 2

@@ -8,11 +8,12 @@
 // of host threads each take the next piece and copy it between the caller's
 // array and its buffer, and the calling thread issues the DMAs between its own
 // pieces, so host copies and DMA overlap and the copy runs near the PCIe rate.
-// The threads are woken once per copy, one waking the next, and the caller
-// starts at once: waking all of them for every 8 MiB
-// chunk, and waiting for the slowest of them at its end, cost more than the
-// copy itself up to tens of MB (13 MB: 1.63 -> 0.6-0.8 ms, 34 MB: 1.82 -> 1.4-1.6, the
-// driver's own path 0.67 and 1.74; 102 MB 3.6 -> 3.4-3.9).  Pinned
+// The threads are woken once per copy, one waking the next, and the caller starts
+// at once: waking all of them for every 8 MiB chunk, and waiting for the slowest of
+// them at its end, cost more than the copy itself up to tens of MB (that way ->
+// now, in brackets the driver's own: 4 MB 0.6 -> 0.3 ms (0.25), 13 MB 1.5 -> 0.8
+// (0.7), 34 MB 2.0 -> 1.6 (2.9), 102 MB 3.7 -> 3.7 (9.0), 400 MB 9.3 -> 9.2 (35);
+// samples and labels of 5M tets to the host 1.6 -> 1.4, of 80M 31 -> 23).  Pinned
 // source/destination arrays skip the staging.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -37,7 +38,8 @@ namespace gpupr {
 namespace {
 
 constexpr size_t kPiece = 1u << 20;     // bytes per staging buffer
-constexpr int kSlots = 32;              // staging buffers per set
+constexpr int kSlots = 32;              // staging buffers per set, side by side
+constexpr int kGroup = 4;               // pieces one DMA takes in the middle of a copy
 constexpr size_t kDirect = 1u << 20;    // below this, the driver's own path
 
 // A copy's pieces, shared by its caller and the host threads that help it.  A
@@ -158,7 +160,8 @@ struct Staging {
     std::mutex mu;
     char* pin = nullptr;
     cudaEvent_t ev[kSlots] = {};
-    bool pending[kSlots] = {};
+    bool pending[kSlots] = {};   // a DMA of the buffer was issued ...
+    int last[kSlots] = {};       // ... together with the next ones up to this, whose event it has
 };
 
 // Staging sets per device and direction (0 = to device, 1 = to host) that
@@ -212,7 +215,7 @@ void settle(Staging& st)
 {
     for (int k = 0; k < kSlots; ++k)
         if (st.pending[k]) {
-            GPUPR_CUDA(cudaEventSynchronize(st.ev[k]));
+            GPUPR_CUDA(cudaEventSynchronize(st.ev[st.last[k]]));
             st.pending[k] = false;
         }
 }
@@ -229,22 +232,43 @@ bool is_pinned(const void* p)
 
 // Host threads that help the caller with a memcpy through the staging: waking a
 // sleeping thread costs about what copying 1 MiB does, so each has to bring
-// several pieces' worth.  Measured with 0 / 1 / 2 / 3 / 6 helpers: 8 MB 0.62 / 0.36
-// / 0.33 / 0.34 / 0.99 ms, 13 MB 1.0 / 0.56 / 0.75 / 0.91 / 1.19, 34 MB 3.4 / 1.75 /
-// 1.66 / 1.28 / 1.97, 102 MB 11.9 / 6.2 / 4.5 / 3.8 / 3.4.
-int64_t copy_helpers(size_t bytes)
+// several pieces' worth.  To the device, with 0 / 1 / 2 / 3 / 8 helpers at most: 34 MB
+// 2.8 / 2.7 / 1.4 / 1.5 / 1.5 ms, 102 MB 8.3 / 7.9 / 3.3 / 3.0 / 3.8, 400 MB 33 / 18 /
+// 11.5 / 9.1 / 9.2 (four: 2.9-3.4 and 8.5-11, by host).  A larger copy to the host
+// meets pages of the caller's array that were never touched, which its threads
+// fault in side by side: with a helper for 10 / 3 MB of it, samples and labels of 13M
+// tets (52 + 13 MB) took 5.4 / 3.7 ms, of 5M 1.8 / 1.35, but of 3M 1.1 / 1.4 and of 2M
+// 0.9 / 1.0.
+int64_t copy_helpers(size_t bytes, bool to_host)
 {
-    return bytes < (4u << 20) ? 0 : std::max<int64_t>(1, (int64_t)(bytes / (10u << 20)));
+    const size_t each = to_host && bytes >= (16u << 20) ? 3u << 20 : 10u << 20;
+    return bytes < (4u << 20) ? 0 : std::max<int64_t>(1, (int64_t)(bytes / each));
 }
 
-// Issues the DMA of piece p's buffer to the device.
-cudaError_t send(Staging& st, int64_t p, void* d_dst, size_t len, cudaStream_t s)
+// Issues one DMA for the n pieces from p on, whose buffers lie side by side.
+cudaError_t transfer(Staging& st, int64_t p, int64_t n, char* dev, size_t bytes, cudaMemcpyKind kind, cudaStream_t s)
 {
-    const int k = (int)(p % kSlots);
-    const cudaError_t e = cudaMemcpyAsync(d_dst, st.pin + (size_t)k * kPiece, len, cudaMemcpyHostToDevice, s);
+    const int k = (int)(p % kSlots), last = k + (int)n - 1;
+    const size_t off = (size_t)p * kPiece, len = std::min((size_t)n * kPiece, bytes - off);
+    char* pin = st.pin + (size_t)k * kPiece;
+    const cudaError_t e = kind == cudaMemcpyHostToDevice ? cudaMemcpyAsync(dev + off, pin, len, kind, s)
+                                                         : cudaMemcpyAsync(pin, dev + off, len, kind, s);
     if (e != cudaSuccess) return e;
-    st.pending[k] = true;
-    return cudaEventRecord(st.ev[k], s);
+    for (int i = k; i <= last; ++i) {
+        st.pending[i] = true;
+        st.last[i] = last;
+    }
+    return cudaEventRecord(st.ev[last], s);
+}
+
+// Pieces that the next DMA, from piece p on, should wait for: single ones at the
+// ends of a copy, where the link or the caller waits for each; groups between,
+// because each DMA with its event costs the link time of its own (400 MB in
+// single ones 10.2-10.6 ms, in groups of four 9.1-9.5, of eight 9.2-9.5).
+int64_t group_at(int64_t p, int64_t parts)
+{
+    if (p < 2 * kGroup || parts - p <= 2 * kGroup) return 1;
+    return std::min<int64_t>(kGroup, kSlots - p % kSlots);
 }
 
 // The caller works on a piece in this many bytes at a time, so that pieces its
@@ -254,7 +278,7 @@ constexpr size_t kCallerStep = 256u << 10;
 // Runs a copy of `bytes` bytes, in pieces of kPiece,
 // through a staging set: fill(pin, offset, length) copies between a buffer and
 // the caller's array, on this thread or a helper's, once the buffer's last DMA is
-// through; after(p) issues the DMA that follows piece p, in order of the pieces.
+// through; after(p, n) issues the DMA that follows the n pieces from p on, in order.
 // All CUDA calls are this thread's.  After an error nothing more is copied and,
 // once no helper works on the job, the error is thrown.
 template <class After>
@@ -271,9 +295,14 @@ void run_pieces(Staging& st, size_t bytes, int64_t helpers,
     int64_t open = 0;     // job->open
     const int64_t ahead = 1 + copy_pool().enlist(job, helpers);   // pieces asked for at once
     auto pass = [&] {
-        while (err == cudaSuccess && passed < parts &&
-               job->done[passed % kSlots].load(std::memory_order_acquire) == passed + 1)
-            err = after(passed++);
+        while (err == cudaSuccess && passed < parts) {
+            const int64_t most = std::min(std::min<int64_t>(kGroup, kSlots - passed % kSlots), parts - passed);
+            int64_t n = 0;
+            while (n < most && job->done[(passed + n) % kSlots].load(std::memory_order_acquire) == passed + n + 1) ++n;
+            if (n < group_at(passed, parts)) return;
+            err = after(passed, n);
+            passed += n;
+        }
     };
     // a buffer opens when its last DMA is through: waited for only when a piece
     // in it is asked for, or may be next
@@ -282,7 +311,7 @@ void run_pieces(Staging& st, size_t bytes, int64_t helpers,
         while (err == cudaSuccess && open < want) {
             const int k = (int)(open % kSlots);
             if (st.pending[k]) {
-                err = cudaEventSynchronize(st.ev[k]);
+                err = cudaEventSynchronize(st.ev[st.last[k]]);
                 if (err != cudaSuccess) return;
                 st.pending[k] = false;
             }
@@ -328,12 +357,9 @@ void host_to_device(void* d_dst, const void* h_src, size_t bytes, cudaStream_t s
     const char* src = static_cast<const char*>(h_src);
     char* dst = static_cast<char*>(d_dst);
     run_pieces(
-        st, bytes, copy_helpers(bytes),
+        st, bytes, copy_helpers(bytes, false),
         [&](char* pin, size_t off, size_t len) { std::memcpy(pin, src + off, len); },
-        [&](int64_t p) {
-            const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
-            return send(st, p, dst + off, len, s);
-        });
+        [&](int64_t p, int64_t n) { return transfer(st, p, n, dst, bytes, cudaMemcpyHostToDevice, s); });
 }
 
 void device_to_host(void* h_dst, const void* d_src, size_t bytes, cudaStream_t s)
@@ -347,25 +373,23 @@ void device_to_host(void* h_dst, const void* d_src, size_t bytes, cudaStream_t s
     StagingLease lease = staging(1);
     Staging& st = *lease.st;
     settle(st);
-    const char* src = static_cast<const char*>(d_src);
+    char* src = static_cast<char*>(const_cast<void*>(d_src));
     char* dst = static_cast<char*>(h_dst);
-    const int64_t pieces = (int64_t)((bytes + kPiece - 1) / kPiece);
-    auto issue = [&](int64_t p) {
-        const int k = (int)(p % kSlots);
-        const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
-        const cudaError_t e = cudaMemcpyAsync(st.pin + (size_t)k * kPiece, src + off, len,
-                                              cudaMemcpyDeviceToHost, s);
-        if (e != cudaSuccess) return e;
-        st.pending[k] = true;
-        return cudaEventRecord(st.ev[k], s);
-    };
-    // a ring of DMAs ahead; once a piece is copied out, the one that follows in
-    // its buffer is issued
-    for (int64_t p = 0; p < std::min<int64_t>(pieces, kSlots); ++p) GPUPR_CUDA(issue(p));
+    const int64_t parts = (int64_t)((bytes + kPiece - 1) / kPiece);
+    auto issue = [&](int64_t p, int64_t n) { return transfer(st, p, n, src, bytes, cudaMemcpyDeviceToHost, s); };
+    // a ring of DMAs ahead; once pieces are copied out, those that follow in
+    // their buffers are issued
+    for (int64_t p = 0, n; p < std::min<int64_t>(parts, kSlots); p += n) {
+        n = group_at(p, parts);
+        GPUPR_CUDA(issue(p, n));
+    }
     run_pieces(
-        st, bytes, copy_helpers(bytes),
+        st, bytes, copy_helpers(bytes, true),
         [&](char* pin, size_t off, size_t len) { std::memcpy(dst + off, pin, len); },
-        [&](int64_t p) { return p + kSlots < pieces ? issue(p + kSlots) : cudaSuccess; });
+        [&](int64_t p, int64_t n) {
+            const int64_t q = p + kSlots;
+            return q < parts ? issue(q, std::min(n, parts - q)) : cudaSuccess;
+        });
 }
 
 // Nx4 integer topology (int32 or int64 elements, any byte strides, e.g. a
@@ -407,10 +431,7 @@ void upload_topology(int32_t* d_out, const void* host, uint64_t rows, int64_t ro
                 }
             }
         },
-        [&](int64_t p) {
-            const size_t off = (size_t)p * kPiece, len = std::min(kPiece, bytes - off);
-            return send(st, p, dst + off, len, s);
-        });
+        [&](int64_t p, int64_t n) { return transfer(st, p, n, dst, bytes, cudaMemcpyHostToDevice, s); });
 }
 
 namespace {
